@@ -221,7 +221,8 @@ int omr_ntt_plan_passes(int field, uint32_t log_n, int plan, uint64_t batch, uin
  * the pass's buffer roles bound to `src` (source), `scratch` (N * batch words,
  * caller-owned) and `dst` (destination).  Running every pass in order equals
  * omr_ntt_forward / omr_ntt_inverse; used to time and tune passes one at a
- * time.  No reference counterpart (the reference has no pass structure). */
+ * time.  The words in `scratch` between passes are internal: Goldilocks ones
+ * are any u64 congruent to the value.  No reference counterpart (the reference has no pass structure). */
 int omr_ntt_plan_run_pass(omr_ntt_domain_t d, int plan, int pass, int inverse, const void *src,
                           void *scratch, void *dst, uint64_t batch, void *stream);
 

@@ -194,7 +194,7 @@ OMR_D void batch_row_tile(const BatchArgs& ba, const BatchReq& r, uint32_t g, ty
       K = (n - K) & (n - 1);
       y = F::mul_tw(y, scale);
     }
-    dst[K] = y;
+    dst[K] = F::canon(y);
   }
 }
 

@@ -25,6 +25,7 @@
 #pragma once
 #include <cstdint>
 
+#include "dft_goldilocks.cuh"
 #include "fields.cuh"
 
 namespace omr {
@@ -110,13 +111,9 @@ struct RootConst {
   static constexpr typename F::Tw tw = F::make_tw(value);
 };
 
-// Goldilocks: 2 has order 192 (2^96 = -1), and omega_64 = 7^((p-1)/64) = 2^39,
-// so omega_R^k = 2^(39 (64/R) k mod 192) for R <= 64.
-constexpr int gl_root_exp(int logr, int k) { return (39 * (64 >> logr) * k) % 192; }
-
-// In-register R-point DFT (R = 2^LOGR), natural order in and out.
-// Radix-2 decimation in frequency: (u + v, (u - v) * omega_len^j), outputs in
-// bit-reversed register order, undone by compile-time renaming.
+// In-register R-point DFT (R = 2^LOGR) of the 32-bit fields, natural order in
+// and out.  Radix-2 decimation in frequency: (u + v, (u - v) * omega_len^j),
+// outputs in bit-reversed register order, undone by compile-time renaming.
 template <class F, int LOGR, bool INV, int LEN_LOG, int BLK, int J>
 OMR_D void dif_stage_bf(typename F::E* v) {
   constexpr int HALF = 1 << (LEN_LOG - 1);
@@ -129,18 +126,8 @@ OMR_D void dif_stage_bf(typename F::E* v) {
     constexpr int K = J << (LOGR - LEN_LOG);
     constexpr int R = 1 << LOGR;
     constexpr int KK = INV ? ((R - K) % R) : K;
-    if constexpr (F::ID == GOLDILOCKS && LOGR <= 6) {
-      // omega_R^KK = 2^E: a shift-and-fold multiply; 2^(E - 96) = -2^E swaps the difference
-      constexpr int E = gl_root_exp(LOGR, KK);
-      static_assert(hpowmod(2, E, F::p64()) == RootConst<F, LOGR, KK>::value, "root as a power of 2");
-      if constexpr (E >= 96)
-        v[BLK + J + HALF] = F::template mul_pow2<E - 96>(F::sub(w, u));
-      else
-        v[BLK + J + HALF] = F::template mul_pow2<E>(F::sub(u, w));
-    } else {
-      constexpr typename F::Tw t = RootConst<F, LOGR, KK>::tw;
-      v[BLK + J + HALF] = F::mul_tw(sub_lazy<F>(u, w), t);
-    }
+    constexpr typename F::Tw t = RootConst<F, LOGR, KK>::tw;
+    v[BLK + J + HALF] = F::mul_tw(sub_lazy<F>(u, w), t);
   }
 }
 
@@ -170,16 +157,48 @@ constexpr int bitrev_c(int x, int bits) {
   return r;
 }
 
+// In-register R-point DFT, natural order in and out.  32-bit fields: canonical
+// in and out.  Goldilocks: any u64 in and out, on
+// three-limb values in between (dft_goldilocks.cuh).
 template <class F, int LOGR, bool INV>
 OMR_D void dft_reg(typename F::E (&v)[1 << LOGR]) {
   constexpr int R = 1 << LOGR;
   using E = typename F::E;
-  dif_stages<F, LOGR, INV, LOGR>(v);
-  E t[R];
+  if constexpr (F::ID == GOLDILOCKS) {
+    GlWide g[R];
 #pragma unroll
-  for (int k = 0; k < R; k++) t[k] = v[k];
+    for (int k = 0; k < R; k++) g[k] = gl_wide(v[k]);
+    gl_dft3<LOGR, INV>(g);
 #pragma unroll
-  for (int k = 0; k < R; k++) v[k] = t[bitrev_c(k, LOGR)];
+    for (int k = 0; k < R; k++) v[k] = gl_fold(g[k]);
+  } else {
+    dif_stages<F, LOGR, INV, LOGR>(v);
+    E t[R];
+#pragma unroll
+    for (int k = 0; k < R; k++) t[k] = v[k];
+#pragma unroll
+    for (int k = 0; k < R; k++) v[k] = t[bitrev_c(k, LOGR)];
+  }
+}
+
+// The same on twiddled inputs, v[q] tw(q) for q >= 1.  Goldilocks products
+// enter the DFT unreduced, so one fold per element is saved.
+template <class F, int LOGR, bool INV, class TwOf>
+OMR_D void dft_reg_tw(typename F::E (&v)[1 << LOGR], TwOf&& tw) {
+  constexpr int R = 1 << LOGR;
+  if constexpr (F::ID == GOLDILOCKS) {
+    GlWide g[R];
+    g[0] = gl_wide(v[0]);
+#pragma unroll
+    for (int q = 1; q < R; q++) g[q] = F::mul3(v[q], tw(q).w);
+    gl_dft3<LOGR, INV>(g);
+#pragma unroll
+    for (int k = 0; k < R; k++) v[k] = gl_fold(g[k]);
+  } else {
+#pragma unroll
+    for (int q = 1; q < R; q++) v[q] = F::mul_tw(v[q], tw(q));
+    dft_reg<F, LOGR, INV>(v);
+  }
 }
 
 // Shared-memory tile [T rows][C cols] with an XOR swizzle so that both a
@@ -205,9 +224,9 @@ struct RoundPlan {
 };
 
 // Radix 16 for every field.  For Goldilocks omega_16 = -2^60, so all of a
-// round's in-register twiddles are shift-and-fold multiplies; 3 rounds of a
+// round's in-register twiddles are shifts (dft_goldilocks.cuh); 3 rounds of a
 // 4096-point line (instead of 4 of radix 8) drop a twiddle boundary and an
-// exchange, and 16 u64 words per thread still fit without spills.
+// exchange.
 template <class F>
 constexpr int max_radix_log() {
   return 4;
@@ -281,11 +300,10 @@ OMR_D void do_round(const PassArgs<F>& a, typename F::E* s, const typename F::E*
       if constexpr (LOGNS > 0) {
         // a_q *= omega_{NS*R}^{q*jm} = omega_T^{q*jm*T/(NS*R)}
         constexpr int SCALE = T / (NS * R);
-#pragma unroll
-        for (int q = 1; q < R; q++)
-          v[i][q] = F::mul_tw(v[i][q], a.roots[(uint32_t)(q * jm * SCALE) * a.roots_stride]);
+        dft_reg_tw<F, LOGR, INV>(v[i], [&](int q) { return a.roots[(uint32_t)(q * jm * SCALE) * a.roots_stride]; });
+      } else {
+        dft_reg<F, LOGR, INV>(v[i]);
       }
-      dft_reg<F, LOGR, INV>(v[i]);
       const int d = ((j >> LOGNS) << (LOGNS + LOGR)) | jm;
       // four-step twiddle of output k = d + q NS: omega_N^(line k scale) =
       // base * step^q, base = omega_N^(line d scale), step = omega_N^(line NS
@@ -326,6 +344,7 @@ OMR_D void do_round(const PassArgs<F>& a, typename F::E* s, const typename F::E*
               }
             }
             if (a.has_scale) y = F::mul_tw(y, a.scale);
+            if constexpr (!TW) y = F::canon(y);  // the transform's result
             if constexpr (JF)
               gout[(uint64_t)c * a.os_lo + (uint32_t)k] = y;
             else

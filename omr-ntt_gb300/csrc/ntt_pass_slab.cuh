@@ -258,11 +258,15 @@ OMR_D void slab_rounds12(const PassArgs<F>& a, unsigned char* s, const typename 
   __syncwarp();
 #pragma unroll
   for (int c = 0; c < VPU; c++) dft_reg<F, 4, INV>(v[c]);
+  // twiddle omega_256^(l a): Goldilocks multiplies after the exchange, where
+  // the products enter the second DFT unreduced
+  if constexpr (F::ID != GOLDILOCKS) {
 #pragma unroll
-  for (int aa = 1; aa < 16; aa++) {
-    const typename F::Tw t = tab1[(aa - 1) * 16 + l];
+    for (int aa = 1; aa < 16; aa++) {
+      const typename F::Tw t = tab1[(aa - 1) * 16 + l];
 #pragma unroll
-    for (int c = 0; c < VPU; c++) v[c][aa] = F::mul_tw(v[c][aa], t);
+      for (int c = 0; c < VPU; c++) v[c][aa] = F::mul_tw(v[c][aa], t);
+    }
   }
   // exchange: V[l][a] to row 16 a + (l ^ a)
 #pragma unroll
@@ -284,7 +288,12 @@ OMR_D void slab_rounds12(const PassArgs<F>& a, unsigned char* s, const typename 
   }
   __syncwarp();
 #pragma unroll
-  for (int c = 0; c < VPU; c++) dft_reg<F, 4, INV>(v[c]);
+  for (int c = 0; c < VPU; c++) {
+    if constexpr (F::ID == GOLDILOCKS)
+      dft_reg_tw<F, 4, INV>(v[c], [&](int ll) { return tab1[(ll - 1) * 16 + am]; });
+    else
+      dft_reg<F, 4, INV>(v[c]);
+  }
   // outputs b = 0..15 are line entries kk = k1 + R0 (am + 16 b)
   if constexpr (TW) {
 #pragma unroll
@@ -307,6 +316,12 @@ OMR_D void slab_rounds12(const PassArgs<F>& a, unsigned char* s, const typename 
     for (int c = 0; c < VPU; c++)
 #pragma unroll
       for (int b = 0; b < 16; b++) v[c][b] = F::mul_tw(v[c][b], a.scale);
+  }
+  if constexpr (MODE != MODE_COL) {  // the transform's results
+#pragma unroll
+    for (int c = 0; c < VPU; c++)
+#pragma unroll
+      for (int b = 0; b < 16; b++) v[c][b] = F::canon(v[c][b]);
   }
   // staging rows a + 16 b, interleaved columns (both modes)
 #pragma unroll

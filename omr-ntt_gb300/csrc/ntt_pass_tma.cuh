@@ -251,10 +251,10 @@ OMR_D void tma_round(const PassArgs<F>& a, const SmemTw<F>& st, typename F::E* s
       const int jm = j & (NS - 1);
       if constexpr (LOGNS > 0) {
         const typename F::Tw* tw = st.rtw + rtw_off<LOGT, max_radix_log<F>()>(RI) + jm;
-#pragma unroll
-        for (int q = 1; q < R; q++) v[i][q] = F::mul_tw(v[i][q], tw[q * NS]);
+        dft_reg_tw<F, LOGR, INV>(v[i], [&](int q) { return tw[q * NS]; });
+      } else {
+        dft_reg<F, LOGR, INV>(v[i]);
       }
-      dft_reg<F, LOGR, INV>(v[i]);
       const int d = ((j >> LOGNS) << (LOGNS + LOGR)) | jm;
       if constexpr (!LAST) {
 #pragma unroll
@@ -280,6 +280,10 @@ OMR_D void tma_round(const PassArgs<F>& a, const SmemTw<F>& st, typename F::E* s
         if (a.has_scale) {
 #pragma unroll
           for (int q = 0; q < R; q++) v[i][q] = F::mul_tw(v[i][q], a.scale);
+        }
+        if constexpr (!TW) {  // the transform's results
+#pragma unroll
+          for (int q = 0; q < R; q++) v[i][q] = F::canon(v[i][q]);
         }
 #pragma unroll
         for (int q = 0; q < R; q++) s[sidx<F, LOGT, C, STAGE>(d + q * NS, c)] = v[i][q];

@@ -195,11 +195,15 @@ OMR_D void wide_lines(const PassArgs<F>& a, unsigned char* s, const typename F::
   __syncwarp();
 #pragma unroll
   for (int c = 0; c < VPU; c++) dft_reg<F, 4, INV>(v[c]);
+  // twiddle omega_256^(l a): Goldilocks multiplies after the exchange, where
+  // the products enter the second DFT unreduced
+  if constexpr (F::ID != GOLDILOCKS) {
 #pragma unroll
-  for (int aa = 1; aa < 16; aa++) {
-    const typename F::Tw t = tab1[(aa - 1) * 16 + l];
+    for (int aa = 1; aa < 16; aa++) {
+      const typename F::Tw t = tab1[(aa - 1) * 16 + l];
 #pragma unroll
-    for (int c = 0; c < VPU; c++) v[c][aa] = F::mul_tw(v[c][aa], t);
+      for (int c = 0; c < VPU; c++) v[c][aa] = F::mul_tw(v[c][aa], t);
+    }
   }
 #pragma unroll
   for (int aa = 0; aa < 16; aa++) {
@@ -219,7 +223,12 @@ OMR_D void wide_lines(const PassArgs<F>& a, unsigned char* s, const typename F::
   }
   __syncwarp();
 #pragma unroll
-  for (int c = 0; c < VPU; c++) dft_reg<F, 4, INV>(v[c]);
+  for (int c = 0; c < VPU; c++) {
+    if constexpr (F::ID == GOLDILOCKS)
+      dft_reg_tw<F, 4, INV>(v[c], [&](int ll) { return tab1[(ll - 1) * 16 + am]; });
+    else
+      dft_reg<F, 4, INV>(v[c]);
+  }
   // outputs b = 0..15 are line entries am + 16 b
   if (TW && a.tw_tab != nullptr) {
     // twiddle table [line][k]: one operand per output (tw_line_mul_m == 0)
@@ -251,6 +260,12 @@ OMR_D void wide_lines(const PassArgs<F>& a, unsigned char* s, const typename F::
     for (int c = 0; c < VPU; c++)
 #pragma unroll
       for (int b = 0; b < 16; b++) v[c][b] = F::mul_tw(v[c][b], a.scale);
+  }
+  if constexpr (MODE != MODE_COL) {  // the transform's results
+#pragma unroll
+    for (int c = 0; c < VPU; c++)
+#pragma unroll
+      for (int b = 0; b < 16; b++) v[c][b] = F::canon(v[c][b]);
   }
   if constexpr (ROWS) {
 #pragma unroll

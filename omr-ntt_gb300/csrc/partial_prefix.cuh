@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(prefix_threads<F, LOGT>(), 2)
           const Tw z = zi_s[k];
           const int row = (int)(out_index(k) & (uint32_t)(T - 1));
 #pragma unroll
-          for (int c = 0; c < C; c++) h = F::add(F::mul_tw(h, z), s[tile_idx<F, C>(row, c)]);
+          for (int c = 0; c < C; c++) h = F::mul_add(h, z, s[tile_idx<F, C>(row, c)]);
           acc_s[k] = h;
         }
       }
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(prefix_threads<F, LOGT>(), 2)
     if (!many && active) {
 #pragma unroll 4
       for (uint32_t c = slice; c < (uint32_t)C; c += tpk)
-        acc = F::add(F::mul_tw(acc, zi), s[tile_idx<F, C>(rowb, (int)c)]);
+        acc = F::mul_add(acc, zi, s[tile_idx<F, C>(rowb, (int)c)]);
     }
     __syncthreads();  // the next group's first round overwrites the tile
   }
@@ -163,13 +163,13 @@ __global__ void __launch_bounds__(prefix_threads<F, LOGT>(), 2)
       const uint64_t r_last = (uint64_t)(g1 - 1) * C + (C - 1);
       for (uint32_t k = threadIdx.x; k < m; k += NT)
         partial[(uint64_t)blockIdx.x * m + k] =
-            g1 > g0 && in_range(k) ? mul_m<F>(acc_s[k], omega_m<F>(a, r_last * out_index(k))) : (E)0;
+            g1 > g0 && in_range(k) ? F::canon(mul_m<F>(acc_s[k], omega_m<F>(a, r_last * out_index(k)))) : (E)0;
       return;
     }
   }
   if (g1 > g0 && active) {
     const uint64_t r_last = (uint64_t)(g1 - 1) * C + (C - tpk) + slice;
-    acc = in_range(kbase) ? mul_m<F>(acc, omega_m<F>(a, r_last * jb)) : (E)0;
+    acc = in_range(kbase) ? F::canon(mul_m<F>(acc, omega_m<F>(a, r_last * jb))) : (E)0;
   }
   if (tpk > 1) {
     // combine the slices of every output: s[slice * kact + k]
