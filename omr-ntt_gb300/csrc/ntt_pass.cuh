@@ -114,14 +114,22 @@ struct RootConst {
 // In-register R-point DFT (R = 2^LOGR) of the 32-bit fields, natural order in
 // and out.  Radix-2 decimation in frequency: (u + v, (u - v) * omega_len^j),
 // outputs in bit-reversed register order, undone by compile-time renaming.
-template <class F, int LOGR, bool INV, int LEN_LOG, int BLK, int J>
+// LAZY leaves the last stage's sums and differences of a 31-bit field in
+// [0, 2p): operands of a product only (Shoup and Montgomery take any u32).
+template <class F, int LOGR, bool INV, bool LAZY, int LEN_LOG, int BLK, int J>
 OMR_D void dif_stage_bf(typename F::E* v) {
   constexpr int HALF = 1 << (LEN_LOG - 1);
   using E = typename F::E;
   E u = v[BLK + J], w = v[BLK + J + HALF];
-  v[BLK + J] = F::add(u, w);
+  if constexpr (LAZY && F::SMALL && LEN_LOG == 1)
+    v[BLK + J] = u + w;
+  else
+    v[BLK + J] = F::add(u, w);
   if constexpr (J == 0) {
-    v[BLK + J + HALF] = F::sub(u, w);
+    if constexpr (LAZY && LEN_LOG == 1)
+      v[BLK + J + HALF] = sub_lazy<F>(u, w);
+    else
+      v[BLK + J + HALF] = F::sub(u, w);
   } else {
     constexpr int K = J << (LOGR - LEN_LOG);
     constexpr int R = 1 << LOGR;
@@ -131,23 +139,23 @@ OMR_D void dif_stage_bf(typename F::E* v) {
   }
 }
 
-template <class F, int LOGR, bool INV, int LEN_LOG, int I>
+template <class F, int LOGR, bool INV, bool LAZY, int LEN_LOG, int I>
 OMR_D void dif_stage_iter(typename F::E* v) {
   constexpr int R = 1 << LOGR;
   constexpr int HALF = 1 << (LEN_LOG - 1);
   if constexpr (I < R / 2) {
     constexpr int BLK = (I / HALF) * (2 * HALF);
     constexpr int J = I % HALF;
-    dif_stage_bf<F, LOGR, INV, LEN_LOG, BLK, J>(v);
-    dif_stage_iter<F, LOGR, INV, LEN_LOG, I + 1>(v);
+    dif_stage_bf<F, LOGR, INV, LAZY, LEN_LOG, BLK, J>(v);
+    dif_stage_iter<F, LOGR, INV, LAZY, LEN_LOG, I + 1>(v);
   }
 }
 
-template <class F, int LOGR, bool INV, int LEN_LOG>
+template <class F, int LOGR, bool INV, bool LAZY, int LEN_LOG>
 OMR_D void dif_stages(typename F::E* v) {
   if constexpr (LEN_LOG >= 1) {
-    dif_stage_iter<F, LOGR, INV, LEN_LOG, 0>(v);
-    dif_stages<F, LOGR, INV, LEN_LOG - 1>(v);
+    dif_stage_iter<F, LOGR, INV, LAZY, LEN_LOG, 0>(v);
+    dif_stages<F, LOGR, INV, LAZY, LEN_LOG - 1>(v);
   }
 }
 
@@ -158,9 +166,9 @@ constexpr int bitrev_c(int x, int bits) {
 }
 
 // In-register R-point DFT, natural order in and out.  32-bit fields: canonical
-// in and out.  Goldilocks: any u64 in and out, on
+// in, canonical out (but see LAZY above).  Goldilocks: any u64 in and out, on
 // three-limb values in between (dft_goldilocks.cuh).
-template <class F, int LOGR, bool INV>
+template <class F, int LOGR, bool INV, bool LAZY = false>
 OMR_D void dft_reg(typename F::E (&v)[1 << LOGR]) {
   constexpr int R = 1 << LOGR;
   using E = typename F::E;
@@ -172,7 +180,7 @@ OMR_D void dft_reg(typename F::E (&v)[1 << LOGR]) {
 #pragma unroll
     for (int k = 0; k < R; k++) v[k] = gl_fold(g[k]);
   } else {
-    dif_stages<F, LOGR, INV, LOGR>(v);
+    dif_stages<F, LOGR, INV, LAZY, LOGR>(v);
     E t[R];
 #pragma unroll
     for (int k = 0; k < R; k++) t[k] = v[k];
@@ -181,9 +189,17 @@ OMR_D void dft_reg(typename F::E (&v)[1 << LOGR]) {
   }
 }
 
-// The same on twiddled inputs, v[q] tw(q) for q >= 1.  Goldilocks products
+// A DFT with results 1 .. R - 1 left lazy for a product (result 0, whose
+// twiddle is 1, is reduced).
+template <class F, int LOGR, bool INV>
+OMR_D void dft_reg_mul(typename F::E (&v)[1 << LOGR]) {
+  dft_reg<F, LOGR, INV, true>(v);
+  if constexpr (F::SMALL) v[0] = min(v[0], v[0] - F::P);
+}
+
+// A DFT of twiddled inputs, v[q] tw(q) for q >= 1.  Goldilocks products
 // enter the DFT unreduced, so one fold per element is saved.
-template <class F, int LOGR, bool INV, class TwOf>
+template <class F, int LOGR, bool INV, bool LAZY = false, class TwOf>
 OMR_D void dft_reg_tw(typename F::E (&v)[1 << LOGR], TwOf&& tw) {
   constexpr int R = 1 << LOGR;
   if constexpr (F::ID == GOLDILOCKS) {
@@ -197,7 +213,7 @@ OMR_D void dft_reg_tw(typename F::E (&v)[1 << LOGR], TwOf&& tw) {
   } else {
 #pragma unroll
     for (int q = 1; q < R; q++) v[q] = F::mul_tw(v[q], tw(q));
-    dft_reg<F, LOGR, INV>(v);
+    dft_reg<F, LOGR, INV, LAZY>(v);
   }
 }
 

@@ -206,7 +206,7 @@ OMR_D void slab_round0(unsigned char* buf, const typename F::Tw* tab0) {
       }
     }
 #pragma unroll
-    for (int c = 0; c < CPG; c++) dft_reg<F, LR, INV>(v[c]);
+    for (int c = 0; c < CPG; c++) dft_reg_mul<F, LR, INV>(v[c]);
 #pragma unroll
     for (int k1 = 1; k1 < R0; k1++) {
       const typename F::Tw t = tab0[(k1 - 1) * 256 + j];
@@ -257,7 +257,7 @@ OMR_D void slab_rounds12(const PassArgs<F>& a, unsigned char* s, const typename 
   }
   __syncwarp();
 #pragma unroll
-  for (int c = 0; c < VPU; c++) dft_reg<F, 4, INV>(v[c]);
+  for (int c = 0; c < VPU; c++) dft_reg_mul<F, 4, INV>(v[c]);
   // twiddle omega_256^(l a): Goldilocks multiplies after the exchange, where
   // the products enter the second DFT unreduced
   if constexpr (F::ID != GOLDILOCKS) {
@@ -291,8 +291,8 @@ OMR_D void slab_rounds12(const PassArgs<F>& a, unsigned char* s, const typename 
   for (int c = 0; c < VPU; c++) {
     if constexpr (F::ID == GOLDILOCKS)
       dft_reg_tw<F, 4, INV>(v[c], [&](int ll) { return tab1[(ll - 1) * 16 + am]; });
-    else
-      dft_reg<F, 4, INV>(v[c]);
+    else  // column passes and inverse row passes multiply every result
+      dft_reg<F, 4, INV, TW || INV>(v[c]);
   }
   // outputs b = 0..15 are line entries kk = k1 + R0 (am + 16 b)
   if constexpr (TW) {
@@ -311,7 +311,7 @@ OMR_D void slab_rounds12(const PassArgs<F>& a, unsigned char* s, const typename 
       }
     }
   }
-  if (a.has_scale) {
+  if constexpr (INV && !TW) {  // the last pass of an inverse transform
 #pragma unroll
     for (int c = 0; c < VPU; c++)
 #pragma unroll

@@ -251,9 +251,9 @@ OMR_D void tma_round(const PassArgs<F>& a, const SmemTw<F>& st, typename F::E* s
       const int jm = j & (NS - 1);
       if constexpr (LOGNS > 0) {
         const typename F::Tw* tw = st.rtw + rtw_off<LOGT, max_radix_log<F>()>(RI) + jm;
-        dft_reg_tw<F, LOGR, INV>(v[i], [&](int q) { return tw[q * NS]; });
+        dft_reg_tw<F, LOGR, INV, LAST && TW>(v[i], [&](int q) { return tw[q * NS]; });
       } else {
-        dft_reg<F, LOGR, INV>(v[i]);
+        dft_reg<F, LOGR, INV, LAST && TW>(v[i]);
       }
       const int d = ((j >> LOGNS) << (LOGNS + LOGR)) | jm;
       if constexpr (!LAST) {

@@ -194,7 +194,7 @@ OMR_D void wide_lines(const PassArgs<F>& a, unsigned char* s, const typename F::
   }
   __syncwarp();
 #pragma unroll
-  for (int c = 0; c < VPU; c++) dft_reg<F, 4, INV>(v[c]);
+  for (int c = 0; c < VPU; c++) dft_reg_mul<F, 4, INV>(v[c]);
   // twiddle omega_256^(l a): Goldilocks multiplies after the exchange, where
   // the products enter the second DFT unreduced
   if constexpr (F::ID != GOLDILOCKS) {
@@ -226,8 +226,8 @@ OMR_D void wide_lines(const PassArgs<F>& a, unsigned char* s, const typename F::
   for (int c = 0; c < VPU; c++) {
     if constexpr (F::ID == GOLDILOCKS)
       dft_reg_tw<F, 4, INV>(v[c], [&](int ll) { return tab1[(ll - 1) * 16 + am]; });
-    else
-      dft_reg<F, 4, INV>(v[c]);
+    else  // column passes and inverse row passes multiply every result
+      dft_reg<F, 4, INV, TW || INV>(v[c]);
   }
   // outputs b = 0..15 are line entries am + 16 b
   if (TW && a.tw_tab != nullptr) {
@@ -255,7 +255,7 @@ OMR_D void wide_lines(const PassArgs<F>& a, unsigned char* s, const typename F::
       }
     }
   }
-  if (a.has_scale) {
+  if constexpr (INV && !TW) {  // the last pass of an inverse transform
 #pragma unroll
     for (int c = 0; c < VPU; c++)
 #pragma unroll
