@@ -84,10 +84,12 @@ struct Field32 {
   static constexpr uint32_t to_mont_host(uint64_t w) { return (uint32_t)((w << 32) % P_); }
 
 #if defined(__CUDACC__)
+  // s in [0, 2p) -> [0, p): the smaller of s and s - p (mod 2^32), as one
+  // fused add-min (a plain min of two sums compiles to two instructions)
+  OMR_D static E reduce_once(E s) { return __viaddmin_u32(s, 0u - P, s); }
   OMR_D static E add(E a, E b) {
     if constexpr (SMALL) {
-      E s = a + b;
-      return min(s, s - P);
+      return reduce_once(a + b);
     } else {
       E s = a + b;
       return (s < a || s >= P) ? s - P : s;
@@ -95,8 +97,8 @@ struct Field32 {
   }
   OMR_D static E sub(E a, E b) {
     if constexpr (SMALL) {
-      E d = a - b + P;
-      return min(d, d - P);
+      const E d = a - b;  // a borrow leaves d > 2^32 - p, so d + p wraps below it
+      return __viaddmin_u32(d, P, d);
     } else {
       E d = a - b;
       return a < b ? d + P : d;
@@ -115,8 +117,7 @@ struct Field32 {
   OMR_D static E mul_tw(E a, Tw t) {
     if constexpr (SMALL) {
       uint32_t q = __umulhi(a, t.wq);
-      uint32_t r = a * t.w - q * P;  // in [0, 2p)
-      return min(r, r - P);
+      return reduce_once(a * t.w - q * P);  // in [0, 2p)
     } else {
       return mont(a, t.w);
     }

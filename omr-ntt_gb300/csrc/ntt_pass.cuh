@@ -78,9 +78,9 @@ struct PassArgs {
   uint32_t tw_line_mul_m;
   int has_scale;
   Tw scale;  // N^-1 for inverse transforms
-  // optional: the four-step twiddles of the 256-point column passes as one
-  // table [line][k] (tw_line < 2^13, tw_line_mul_m == 0), replacing the
-  // base * step^q chain with one table operand per output
+  // optional: the four-step twiddles of a wide or two-round column pass as
+  // one table [line][k] (tw_line_mul_m == 0), replacing the base * step^q
+  // chain with one table operand per output
   const Tw* tw_tab;
 };
 
@@ -194,7 +194,7 @@ OMR_D void dft_reg(typename F::E (&v)[1 << LOGR]) {
 template <class F, int LOGR, bool INV>
 OMR_D void dft_reg_mul(typename F::E (&v)[1 << LOGR]) {
   dft_reg<F, LOGR, INV, true>(v);
-  if constexpr (F::SMALL) v[0] = min(v[0], v[0] - F::P);
+  if constexpr (F::SMALL) v[0] = F::reduce_once(v[0]);
 }
 
 // A DFT of twiddled inputs, v[q] tw(q) for q >= 1.  Goldilocks products
