@@ -289,7 +289,8 @@ int omr_ntt_run_candidate(omr_ntt_domain_t d, int strategy, int param, int patte
 
 /* Exhaustive autotuner: times every candidate of the planning point on
  * buffers it allocates (seeded random canonical inputs, L2 flushed before each
- * timed run, CUDA events); ms_out[i] = median ms of candidate i over `reps`.
+ * timed run, CUDA events); ms_out[i] = median ms of candidate i over `reps`
+ * runs of one call, or of up to 24 back to back for short candidates.
  * Returns the candidate count.  Setup-time tool: it allocates. */
 int omr_ntt_tune_point(int field, uint32_t log_n, uint64_t batch, int pattern, uint64_t count,
                        int reps, uint64_t seed, float *ms_out, int cap);

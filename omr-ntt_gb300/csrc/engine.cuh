@@ -140,10 +140,10 @@ struct omr_ntt_domain_s {
   std::map<std::pair<void*, int>, omr::Scratch> scratch;  // keyed by (stream, slot)
   std::vector<omr::PlanShape> plans;
   std::map<uint32_t, omr_ntt_domain_s*> subs;  // smaller domains (same field) for partial paths
-  // [line][k] four-step twiddle tables of 256-point column passes (device),
-  // keyed by (inverse, tw_scale, lines); built on first use
+  // [line][k] four-step twiddle tables of column passes (device), keyed by
+  // (inverse, log2 of the line length, tw_scale, lines); built on first use
   std::mutex line_tw_mu;
-  std::map<std::tuple<int, uint64_t, uint32_t>, void*> line_tw;
+  std::map<std::tuple<int, int, uint64_t, uint32_t>, void*> line_tw;
 };
 
 namespace omr {

@@ -49,7 +49,7 @@ OMR_HD int tc_canon(int row, int k) { return (row >> 3) * 1024 + (k >> 3) * 128 
 
 template <class F>
 constexpr size_t tc_smem_bytes() {
-  return (size_t)wide_buf_bytes<F>() + 4 * kTcAVecBytes + kTcBBytes + 15 * 16 * sizeof(typename F::Tw) + 1024;
+  return (size_t)wide_buf_bytes<F, 8>() + 4 * kTcAVecBytes + kTcBBytes + 15 * 16 * sizeof(typename F::Tw) + 1024;
 }
 
 OMR_D uint64_t tc_desc(uint32_t saddr) {
@@ -79,9 +79,9 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   static_assert(F::WORD == 4, "32-bit fields only");
   using E = typename F::E;
   using Tw = typename F::Tw;
-  constexpr int C = wide_cols<F>(), VPU = slab_vpu<F>();
+  constexpr int C = wide_cols<F, 8>(), VPU = slab_vpu<F>();
   constexpr bool ROWS = MODE == MODE_COL;
-  constexpr int BB = wide_buf_bytes<F>();
+  constexpr int BB = wide_buf_bytes<F, 8>();
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   __shared__ __align__(8) uint64_t bars[2];  // [0] tile landed, [1] MMA group done
   __shared__ uint32_t tmem_base;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   const uint32_t tmem = tmem_base;
   bool outstanding = false;
   if (threadIdx.x == 0 && tile < ntiles) {
-    wide_issue_load<F, MODE>(&in_map, a, tile, s, &bars[0]);
+    wide_issue_load<F, 8, MODE>(&in_map, a, tile, s, &bars[0]);
     outstanding = true;
   }
   for (int i = threadIdx.x; i < kTcBBytes / 16; i += kTcThreads)
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 #pragma unroll
       for (int m = 0; m < 16; m++) {
         E t[VPU];
-        wide_load_unit<F, ROWS>(s, l + 16 * m, warp, u, t);
+        wide_load_unit<F, 8, ROWS>(s, l + 16 * m, warp, u, t);
 #pragma unroll
         for (int c = 0; c < VPU; c++) x[c][m] = t[c];
       }
@@ -232,9 +232,9 @@ __global__ void __launch_bounds__(kTcThreads, 2)
           // exchange: V[l][a] to row 16 a + (l ^ a) of the line
           const int r = 16 * aa + (l ^ aa);
           if constexpr (ROWS)
-            *reinterpret_cast<E*>(s + wide_sw(r, line >> 2, (line & 3) * 4)) = y;
+            *reinterpret_cast<E*>(s + wide_sw<8>(r, line >> 2, (line & 3) * 4)) = y;
           else
-            *reinterpret_cast<E*>(s + line * wide_line_bytes<F>() + r * 4) = y;
+            *reinterpret_cast<E*>(s + line * wide_line_bytes<F, 8>() + r * 4) = y;
         }
       }
     }
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 #pragma unroll
       for (int ll = 0; ll < 16; ll++) {
         E t[VPU];
-        wide_load_unit<F, ROWS>(s, 16 * am + (ll ^ am), warp, u, t);
+        wide_load_unit<F, 8, ROWS>(s, 16 * am + (ll ^ am), warp, u, t);
 #pragma unroll
         for (int c = 0; c < VPU; c++) v[c][ll] = t[c];
       }
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
           E t[VPU];
 #pragma unroll
           for (int c = 0; c < VPU; c++) t[c] = v[c][b];
-          wide_store_unit<F, true>(s, am + 16 * b, warp, u, t);
+          wide_store_unit<F, 8, true>(s, am + 16 * b, warp, u, t);
         }
       }
     }
@@ -295,17 +295,17 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         E t[VPU];
 #pragma unroll
         for (int c = 0; c < VPU; c++) t[c] = v[c][bb];
-        wide_store_unit<F, true>(s, (lane & 15) + 16 * bb, warp, lane >> 4, t);
+        wide_store_unit<F, 8, true>(s, (lane & 15) + 16 * bb, warp, lane >> 4, t);
       }
     }
     fence_proxy_async();
     __syncthreads();
     if (threadIdx.x == 0) {
-      wide_issue_store<F, MODE>(&out_map, a, tile, s);
+      wide_issue_store<F, 8, MODE>(&out_map, a, tile, s);
       if (tile + gridDim.x < ntiles) {
         bulk_wait_read_all();
         fence_proxy_async();
-        wide_issue_load<F, MODE>(&in_map, a, tile + gridDim.x, s, &bars[0]);
+        wide_issue_load<F, 8, MODE>(&in_map, a, tile + gridDim.x, s, &bars[0]);
         outstanding = true;
       }
     }

@@ -1,5 +1,5 @@
-// ntt_pass_wide.cuh -- persistent, double-buffered pass of 256-point lines on
-// 128-byte-wide tiles.
+// ntt_pass_wide.cuh -- persistent, double-buffered pass of 64-, 128- and
+// 256-point lines on 128-byte-wide tiles.
 //
 // How fast a four-step pass can move its data depends on the width of its
 // tile rows: on GB300 a copy in the pattern of a column pass (rows 16 KB
@@ -7,24 +7,25 @@
 // 27 us with 64-byte rows and 23 us -- the speed of a contiguous copy -- with
 // 128-byte rows.  A 4096-point line fills 64 KB of shared memory with only 16
 // bytes of lines per row; a 256-point line allows 128 bytes of lines per row
-// in 32 KB.  So this pass takes C = 128 / word lines (32 for the 32-bit
-// fields, 16 for Goldilocks) of 256 points per tile:
+// in 32 KB.  So this pass takes 128 / word lines (32 for the 32-bit fields, 16
+// for Goldilocks) of 256 points per tile, or twice as many (two boxes side by
+// side) of 128 or 64 points:
 //
-//   * column passes: one 2-D TMA box [C lines x 256 rows] per tile, landed
-//     with the 128-byte swizzle (16-byte chunk ch of row r at chunk
+//   * column passes: one 2-D TMA box [128 bytes of lines x T rows] per box,
+//     landed with the 128-byte swizzle (16-byte chunk ch of row r at chunk
 //     ch ^ (r mod 8)), so that with the lane mapping of wide_lane_l /
 //     wide_lane_u every access below is conflict-free;
-//     row passes: one 1-D bulk copy per line into a padded line-major layout;
-//   * warp w owns the 16-byte column group w (4 or 2 lines); its lanes run
-//     the 256-point transforms of those lines as 16 x 16 (radix-16 round,
-//     twiddle omega_256^(l a), exchange through the warp's own column group
-//     with an XOR swizzle and __syncwarp, radix-16 round), then the four-step
-//     twiddle (column passes: one operand per output from the domain's
-//     [line][k] table when the pass has at most 8192 lines, else a
-//     base * step^q chain) and the inverse scale;
-//   * the results go back as 128-byte rows k = a + 16 b (natural order; a
-//     256-point line needs no output permutation) and one 2-D TMA store
-//     writes the tile;
+//     row passes: one 1-D bulk copy per line into a padded line-major layout,
+//     or (wide_line_boxes) TMA boxes of 32 words of every line;
+//   * warp w owns unit w (one or two 16-byte column groups); its lanes run
+//     the line transforms as 16 x 16, 16 x 8 or 8 x 8 (first round, twiddle
+//     omega_T^(l a), exchange through the warp's own column groups with an XOR
+//     swizzle and __syncwarp, second round), then the four-step twiddle
+//     (column passes: one operand per output from the domain's [line][k] table
+//     where launch_pass gives one, else a base * step^q chain) and the inverse
+//     scale;
+//   * the results go back as 128-byte rows k = a + R1 b (natural order) and
+//     one 2-D TMA store per box writes the tile;
 //   * two tile buffers: the next tile lands while this one computes.
 // Per tile that is one CTA barrier for column passes (every warp's results
 // in the buffer before the store) and two for row passes (the lines are
@@ -33,8 +34,8 @@
 // dependent launch) before the first load.  Goldilocks runs the
 // warp-specialised form at the end of this file.
 //
-// The 256-point line transform is the same 16 x 16 split as the slab pass
-// (ntt_pass_slab.cuh), i.e. the reference's four-step decomposition
+// The line transform is the same split as the slab pass (ntt_pass_slab.cuh),
+// i.e. the reference's four-step decomposition
 // (src/encoders/winterfell_four_step.rs:31-81) within a line.
 #pragma once
 #include <cuda.h>
@@ -43,249 +44,323 @@
 
 namespace omr {
 
-template <class F>
+// Line transform T = R1 x L: 16 x 16, 16 x 8 or 8 x 8.
+template <int LOGT>
+constexpr int wide_r1_log() {
+  return LOGT == 6 ? 3 : 4;
+}
+// A tile is one (256 points) or two 128-byte-wide boxes of T rows; a warp's
+// unit is one or two 16-byte column groups of it, so a tile is eight units.
+template <int LOGT>
+constexpr int wide_boxes() {
+  return LOGT == 8 ? 1 : 2;
+}
+template <class F, int LOGT>
 constexpr int wide_cols() {
-  return 128 / F::WORD;  // lines per tile
+  return wide_boxes<LOGT>() * 128 / F::WORD;  // lines per tile
 }
-constexpr int kWideThreads = 256;  // 8 warps: one per 16-byte column group
-template <class F>
+constexpr int kWideThreads = 256;  // 8 warps: one per unit
+// Row passes of 32-bit fields at 64 and 128 points land their lines by TMA in
+// [32-word column box][line] rows of 128 bytes (128-byte swizzle): two to four
+// loads a tile instead of 64 line copies from one thread.  The others copy
+// line by line into padded runs.
+template <class F, int LOGT>
+constexpr bool wide_line_boxes() {
+  return F::WORD == 4 && LOGT < 8;
+}
+template <class F, int LOGT>
 constexpr int wide_line_bytes() {
-  // row-pass line-major layout, padded so that the lines of a unit sit on
-  // other banks: lines 2u + c of the 32-bit fields 8 banks apart (4-byte
-  // accesses, a whole warp at a time), Goldilocks lines 2w + u 16 banks apart
-  // (8-byte accesses, a half-warp of eight l and two u at a time)
-  return 256 * F::WORD + (F::WORD == 8 ? 64 : 32);
+  // line-major layout, padded so that the lines of a unit sit on other
+  // banks: lines 2u + c of the 32-bit fields 8 banks apart (4-byte accesses,
+  // a whole warp at a time), Goldilocks lines u 16 banks apart (8-byte
+  // accesses, a half-warp of eight l and two u at a time)
+  return (1 << LOGT) * F::WORD + (F::WORD == 8 ? 64 : 32);
 }
-template <class F>
+template <class F, int LOGT>
 constexpr int wide_buf_bytes() {  // a 1024-byte multiple (128-byte swizzle atoms)
-  constexpr int a = 256 * 128, b = wide_cols<F>() * wide_line_bytes<F>();
+  constexpr int a = (1 << LOGT) * 128 * wide_boxes<LOGT>(),
+                b = wide_line_boxes<F, LOGT>() ? 0 : wide_cols<F, LOGT>() * wide_line_bytes<F, LOGT>();
   return ((a > b ? a : b) + 1023) / 1024 * 1024;
 }
-template <class F>
+// In-line twiddles omega_T^(l a): [a - 1][l] for the 32-bit fields, which
+// multiply before the exchange, [l - 1][a] for Goldilocks, which does after.
+template <class F, int LOGT>
+constexpr int wide_tab_entries() {
+  constexpr int R1 = 1 << wide_r1_log<LOGT>(), L = (1 << LOGT) / R1;
+  return F::ID == GOLDILOCKS ? (L - 1) * R1 : (R1 - 1) * L;
+}
+template <class F, int LOGT>
 constexpr size_t wide_smem_bytes() {
-  return 2 * (size_t)wide_buf_bytes<F>() + 15 * 16 * sizeof(typename F::Tw) + 1024;
+  return 2 * (size_t)wide_buf_bytes<F, LOGT>() + wide_tab_entries<F, LOGT>() * sizeof(typename F::Tw) + 1024;
+}
+template <class F, int LOGT>
+OMR_D void wide_fill_tab(typename F::Tw* tab1, const PassArgs<F>& a, int nt) {
+  constexpr int R1 = 1 << wide_r1_log<LOGT>(), L = (1 << LOGT) / R1;
+  constexpr int W = F::ID == GOLDILOCKS ? R1 : L;  // table width
+  for (int i = threadIdx.x; i < wide_tab_entries<F, LOGT>(); i += nt)
+    tab1[i] = a.roots[(uint32_t)((i / W + 1) * (i % W)) * a.roots_stride];
 }
 
 // 128-byte-swizzled row layout: byte of (row r, 16-byte chunk ch, offset o)
-OMR_D int wide_sw(int r, int ch, int o) { return r * 128 + ((ch ^ (r & 7)) << 4) + o; }
+template <int LOGT>
+OMR_D int wide_sw(int r, int ch, int o) {
+  return (ch >> 3) * (128 << LOGT) + r * 128 + (((ch ^ r) & 7) << 4) + o;
+}
 
-// Lane -> (l, u) of the line transforms: l = lane bits 0-2 and 4, u = bit 3.
-// The shared-memory pipe serves 8-byte accesses a half-warp at a time, so
-// each half-warp (lanes 0-15, 16-31) holds the eight values of l mod 8 --
-// eight distinct chunk positions of the swizzle, as rows r = l + 16 m,
-// 16 a + (l ^ a) and a + 16 b all have r mod 8 = l mod 8 (^ a) -- and both
+// Lane -> (l, u, g) of the line transforms.  256 points: l = lane bits 0-2 and
+// 4, u = bit 3; shorter lines: l = bits 0-2, u = bit 3, g = bit 4 (the unit's
+// column group).  The shared-memory pipe serves 8-byte accesses a half-warp at
+// a time, so each half-warp (lanes 0-15, 16-31) holds the eight values of l
+// mod 8 -- eight distinct chunk positions of the swizzle, as rows r = l + L m,
+// L a + (l ^ a) and a + R1 b all have r mod 8 = l mod 8 (^ a) -- and both
 // units u: 16 distinct 8-byte slots, one wavefront per half-warp.  (l = lane
 // & 15, u = lane >> 4 put rows r and r + 8 of one unit into the same
 // half-warp: a two-way conflict on every access.)
-OMR_D int wide_lane_l(int lane) { return (lane & 7) | ((lane >> 1) & 8); }
-OMR_D int wide_lane_u(int lane) { return (lane >> 3) & 1; }
-
-// The column unit u (8 bytes) of column group w, row r.
-template <class F, bool ROWS_LAYOUT>
-OMR_D void wide_load_unit(const unsigned char* s, int r, int w, int u, typename F::E* dst) {
-  constexpr int VPU = slab_vpu<F>();
-  if constexpr (ROWS_LAYOUT) {
-    const unsigned char* p = s + wide_sw(r, w, u * 8);
-    if constexpr (F::WORD == 4) {
-      const uint2 x = *reinterpret_cast<const uint2*>(p);
-      dst[0] = x.x;
-      dst[1] = x.y;
-    } else {
-      dst[0] = *reinterpret_cast<const uint64_t*>(p);
-    }
-  } else {  // line-major: line (w * 16 + u * 8) / word + c
-#pragma unroll
-    for (int c = 0; c < VPU; c++)
-      dst[c] = *reinterpret_cast<const typename F::E*>(
-          s + (w * (16 / F::WORD) + u * VPU + c) * wide_line_bytes<F>() + r * F::WORD);
-  }
+template <int LOGT>
+OMR_D int wide_lane_l(int lane) {
+  return LOGT == 8 ? ((lane & 7) | ((lane >> 1) & 8)) : (lane & 7);
 }
-template <class F, bool ROWS_LAYOUT>
-OMR_D void wide_store_unit(unsigned char* s, int r, int w, int u, const typename F::E* src) {
+OMR_D int wide_lane_u(int lane) { return (lane >> 3) & 1; }
+// the lane's 16-byte column group of unit w
+template <int LOGT>
+OMR_D int wide_chunk(int w, int lane) {
+  return LOGT == 8 ? w : 2 * w + (lane >> 4);
+}
+
+// The column unit u (8 bytes) of column group ch, row r.
+template <class F, int LOGT, bool ROWS_LAYOUT>
+OMR_D typename F::E* wide_word(unsigned char* s, int r, int ch, int u, int c) {
+  using E = typename F::E;
+  const int line = ch * (16 / F::WORD) + u * slab_vpu<F>() + c;
+  if constexpr (ROWS_LAYOUT)
+    return reinterpret_cast<E*>(s + wide_sw<LOGT>(r, ch, u * 8 + c * F::WORD));
+  else if constexpr (wide_line_boxes<F, LOGT>())
+    return reinterpret_cast<E*>(s + (r >> 5) * (wide_cols<F, LOGT>() * 128) + line * 128 +
+                                (((r & 31) * 4) ^ ((line & 7) << 4)));
+  else
+    return reinterpret_cast<E*>(s + line * wide_line_bytes<F, LOGT>() + r * F::WORD);
+}
+template <class F, int LOGT, bool ROWS_LAYOUT>
+OMR_D void wide_load_unit(unsigned char* s, int r, int ch, int u, typename F::E* dst) {
   constexpr int VPU = slab_vpu<F>();
-  if constexpr (ROWS_LAYOUT) {
-    unsigned char* p = s + wide_sw(r, w, u * 8);
-    if constexpr (F::WORD == 4)
-      *reinterpret_cast<uint2*>(p) = make_uint2(src[0], src[1]);
-    else
-      *reinterpret_cast<uint64_t*>(p) = src[0];
+  if constexpr (ROWS_LAYOUT && F::WORD == 4) {
+    const uint2 x = *reinterpret_cast<const uint2*>(wide_word<F, LOGT, true>(s, r, ch, u, 0));
+    dst[0] = x.x;
+    dst[1] = x.y;
   } else {
 #pragma unroll
-    for (int c = 0; c < VPU; c++)
-      *reinterpret_cast<typename F::E*>(s + (w * (16 / F::WORD) + u * VPU + c) * wide_line_bytes<F>() +
-                                        r * F::WORD) = src[c];
+    for (int c = 0; c < VPU; c++) dst[c] = *wide_word<F, LOGT, ROWS_LAYOUT>(s, r, ch, u, c);
+  }
+}
+template <class F, int LOGT, bool ROWS_LAYOUT>
+OMR_D void wide_store_unit(unsigned char* s, int r, int ch, int u, const typename F::E* src) {
+  constexpr int VPU = slab_vpu<F>();
+  if constexpr (ROWS_LAYOUT && F::WORD == 4) {
+    *reinterpret_cast<uint2*>(wide_word<F, LOGT, true>(s, r, ch, u, 0)) = make_uint2(src[0], src[1]);
+  } else {
+#pragma unroll
+    for (int c = 0; c < VPU; c++) *wide_word<F, LOGT, ROWS_LAYOUT>(s, r, ch, u, c) = src[c];
   }
 }
 
-template <class F, int MODE>
+OMR_D void tma_load_4d(void* dst, const CUtensorMap* map, int x, int y, int z, int w, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(bar))
+      : "memory");
+}
+
+template <class F, int LOGT, int MODE>
 OMR_D void wide_issue_load(const CUtensorMap* map, const PassArgs<F>& a, uint64_t tile,
                            unsigned char* buf, uint64_t* bar) {
   using E = typename F::E;
-  constexpr int C = wide_cols<F>();
+  constexpr int T = 1 << LOGT, C = wide_cols<F, LOGT>(), BX = wide_boxes<LOGT>();
   uint32_t g, lm;
   uint64_t lb;
   tile_coords<F, C>(a, tile, g, lm, lb);
-  mbar_arrive_expect_tx(bar, (uint32_t)(256 * C * F::WORD));
+  mbar_arrive_expect_tx(bar, (uint32_t)(T * C * F::WORD));
   if constexpr (MODE == MODE_COL) {
-    tma_load_2d(buf, map, (int)(g * C), (int)((lb * a.L_m + lm) * 256ull), bar);
+#pragma unroll
+    for (int b = 0; b < BX; b++)
+      tma_load_2d(buf + b * T * 128, map, (int)(g * C) + b * (C / BX), (int)((lb * a.L_m + lm) * (uint64_t)T), bar);
+  } else if constexpr (wide_line_boxes<F, LOGT>()) {
+#pragma unroll
+    for (int j = 0; j < T / 32; j++)
+      tma_load_4d(buf + j * C * 128, map, 32 * j, (int)(g * C), (int)lm, (int)lb, bar);
   } else {
     const E* src = a.in + (lb * a.is_b + lm * a.is_m + (uint64_t)(g * C) * a.is_lo);
 #pragma unroll 1
     for (int c = 0; c < C; c++)
-      bulk_load(buf + c * wide_line_bytes<F>(), src + (uint64_t)c * a.is_lo, 256 * F::WORD, bar);
+      bulk_load(buf + c * wide_line_bytes<F, LOGT>(), src + (uint64_t)c * a.is_lo, T * F::WORD, bar);
   }
 }
 
-template <class F, int MODE>
+template <class F, int LOGT, int MODE>
 OMR_D void wide_issue_store(const CUtensorMap* map, const PassArgs<F>& a, uint64_t tile,
                             const unsigned char* buf) {
-  constexpr int C = wide_cols<F>();
+  constexpr int T = 1 << LOGT, C = wide_cols<F, LOGT>(), BX = wide_boxes<LOGT>();
   uint32_t g, lm;
   uint64_t lb;
   tile_coords<F, C>(a, tile, g, lm, lb);
-  if constexpr (MODE == MODE_COL)
-    tma_store_2d(map, (int)(g * C), (int)((lb * a.L_m + lm) * 256ull), buf);
-  else
-    tma_store_2d(map, (int)(g * C + lm * (uint32_t)a.os_m), (int)(lb * 256ull), buf);
+#pragma unroll
+  for (int b = 0; b < BX; b++) {
+    if constexpr (MODE == MODE_COL)
+      tma_store_2d(map, (int)(g * C) + b * (C / BX), (int)((lb * a.L_m + lm) * (uint64_t)T), buf + b * T * 128);
+    else
+      tma_store_2d(map, (int)(g * C + lm * (uint32_t)a.os_m) + b * (C / BX), (int)(lb * (uint64_t)T),
+                   buf + b * T * 128);
+  }
   bulk_commit();
 }
 
-// wide_issue_load by a whole warp: the row passes' C line copies go out
+// wide_issue_load by a whole warp: a row pass's C <= 32 line copies go out
 // from C lanes at once (one thread issues a bulk copy in ~70 ns, so C = 32
 // copies from one thread take longer than the tile's compute).  The
-// expect-tx arrive (lane 0) comes first; column passes are one TMA load.
-template <class F, int MODE>
+// expect-tx arrive (lane 0) comes first; column passes are one or two TMA
+// loads.
+template <class F, int LOGT, int MODE>
 OMR_D void wide_issue_load_warp(const CUtensorMap* map, const PassArgs<F>& a, uint64_t tile,
                                 unsigned char* buf, uint64_t* bar, int lane) {
   using E = typename F::E;
-  constexpr int C = wide_cols<F>();
-  if constexpr (MODE == MODE_COL) {
-    if (lane == 0) wide_issue_load<F, MODE>(map, a, tile, buf, bar);
+  constexpr int T = 1 << LOGT, C = wide_cols<F, LOGT>();
+  if constexpr (MODE == MODE_COL || wide_line_boxes<F, LOGT>()) {
+    if (lane == 0) wide_issue_load<F, LOGT, MODE>(map, a, tile, buf, bar);
   } else {
+    static_assert(C <= 32, "one line copy a lane");
     uint32_t g, lm;
     uint64_t lb;
     tile_coords<F, C>(a, tile, g, lm, lb);
-    if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)(256 * C * F::WORD));
+    if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)(T * C * F::WORD));
     __syncwarp();
     const E* src = a.in + (lb * a.is_b + lm * a.is_m + (uint64_t)(g * C) * a.is_lo);
     if (lane < C)
-      bulk_load(buf + lane * wide_line_bytes<F>(), src + (uint64_t)lane * a.is_lo, 256 * F::WORD, bar);
+      bulk_load(buf + lane * wide_line_bytes<F, LOGT>(), src + (uint64_t)lane * a.is_lo, T * F::WORD, bar);
   }
 }
 
-// One warp: the 256-point transforms of column group w.  The results are
-// left in registers, v[c][b] = line entry a + 16 b (a = wide_lane_l(lane)); column
-// passes also write them to the swizzled rows in place, row passes re-lay
-// them as rows after a CTA barrier (their lines span every column group).
-template <class F, int MODE, bool INV, bool TW>
-OMR_D void wide_lines(const PassArgs<F>& a, unsigned char* s, const typename F::Tw* tab1, int w,
-                      uint32_t llo0, uint32_t lm, typename F::E (&v)[slab_vpu<F>()][16]) {
+// Unit w's results (wide_lines) to the swizzled rows.
+template <class F, int LOGT>
+OMR_D void wide_store_rows(unsigned char* s, int w, const typename F::E (&v)[slab_vpu<F>()][1 << wide_r1_log<LOGT>()]) {
   using E = typename F::E;
-  constexpr int VPU = slab_vpu<F>();
+  constexpr int VPU = slab_vpu<F>(), R1 = 1 << wide_r1_log<LOGT>(), L = (1 << LOGT) / R1;
+  const int lane = threadIdx.x & 31;
+  const int am = wide_lane_l<LOGT>(lane), u = wide_lane_u(lane), ch = wide_chunk<LOGT>(w, lane);
+#pragma unroll
+  for (int i = 0; i < R1 / L; i++)
+#pragma unroll
+    for (int b = 0; b < L; b++) {
+      E x[VPU];
+#pragma unroll
+      for (int c = 0; c < VPU; c++) x[c] = v[c][i * L + b];
+      wide_store_unit<F, LOGT, true>(s, am + L * i + R1 * b, ch, u, x);
+    }
+}
+
+// One warp: the line transforms of unit w.  The results are left in
+// registers, v[c][i L + b] = line entry (am + L i) + R1 b (am =
+// wide_lane_l(lane)); column passes also write them to the swizzled rows in
+// place, row passes re-lay them as rows after a CTA barrier (their lines span
+// every unit).
+template <class F, int LOGT, int MODE, bool INV, bool TW>
+OMR_D void wide_lines(const PassArgs<F>& a, unsigned char* s, const typename F::Tw* tab1, int w,
+                      uint32_t llo0, uint32_t lm, typename F::E (&v)[slab_vpu<F>()][1 << wide_r1_log<LOGT>()]) {
+  using E = typename F::E;
+  constexpr int VPU = slab_vpu<F>(), LR1 = wide_r1_log<LOGT>(), R1 = 1 << LR1, LL = LOGT - LR1, L = 1 << LL;
+  constexpr int PER = R1 / L;  // second-round DFTs per line and lane
   constexpr bool ROWS = MODE == MODE_COL;
   const int lane = threadIdx.x & 31;
-  const int l = wide_lane_l(lane), u = wide_lane_u(lane);
+  const int l = wide_lane_l<LOGT>(lane), u = wide_lane_u(lane), ch = wide_chunk<LOGT>(w, lane);
 #pragma unroll
-  for (int m = 0; m < 16; m++) {
+  for (int m = 0; m < R1; m++) {
     E x[VPU];
-    wide_load_unit<F, ROWS>(s, l + 16 * m, w, u, x);
+    wide_load_unit<F, LOGT, ROWS>(s, l + L * m, ch, u, x);
 #pragma unroll
     for (int c = 0; c < VPU; c++) v[c][m] = x[c];
   }
   __syncwarp();
 #pragma unroll
-  for (int c = 0; c < VPU; c++) dft_reg_mul<F, 4, INV>(v[c]);
-  // twiddle omega_256^(l a): Goldilocks multiplies after the exchange, where
+  for (int c = 0; c < VPU; c++) dft_reg_mul<F, LR1, INV>(v[c]);
+  // twiddle omega_T^(l a): Goldilocks multiplies after the exchange, where
   // the products enter the second DFT unreduced
   if constexpr (F::ID != GOLDILOCKS) {
 #pragma unroll
-    for (int aa = 1; aa < 16; aa++) {
-      const typename F::Tw t = tab1[(aa - 1) * 16 + l];
+    for (int aa = 1; aa < R1; aa++) {
+      const typename F::Tw t = tab1[(aa - 1) * L + l];
 #pragma unroll
       for (int c = 0; c < VPU; c++) v[c][aa] = F::mul_tw(v[c][aa], t);
     }
   }
 #pragma unroll
-  for (int aa = 0; aa < 16; aa++) {
+  for (int aa = 0; aa < R1; aa++) {
     E x[VPU];
 #pragma unroll
     for (int c = 0; c < VPU; c++) x[c] = v[c][aa];
-    wide_store_unit<F, ROWS>(s, 16 * aa + (l ^ aa), w, u, x);
+    wide_store_unit<F, LOGT, ROWS>(s, L * aa + (l ^ (aa & (L - 1))), ch, u, x);
   }
   __syncwarp();
   const int am = l;
 #pragma unroll
-  for (int ll = 0; ll < 16; ll++) {
-    E x[VPU];
-    wide_load_unit<F, ROWS>(s, 16 * am + (ll ^ am), w, u, x);
+  for (int i = 0; i < PER; i++)
 #pragma unroll
-    for (int c = 0; c < VPU; c++) v[c][ll] = x[c];
-  }
+    for (int ll = 0; ll < L; ll++) {
+      E x[VPU];
+      wide_load_unit<F, LOGT, ROWS>(s, L * (am + L * i) + (ll ^ am), ch, u, x);
+#pragma unroll
+      for (int c = 0; c < VPU; c++) v[c][i * L + ll] = x[c];
+    }
   __syncwarp();
 #pragma unroll
-  for (int c = 0; c < VPU; c++) {
-    if constexpr (F::ID == GOLDILOCKS)
-      dft_reg_tw<F, 4, INV>(v[c], [&](int ll) { return tab1[(ll - 1) * 16 + am]; });
-    else  // column passes and inverse row passes multiply every result
-      dft_reg<F, 4, INV, TW || INV>(v[c]);
-  }
-  // outputs b = 0..15 are line entries am + 16 b
-  if (TW && a.tw_tab != nullptr) {
-    // twiddle table [line][k]: one operand per output (tw_line_mul_m == 0)
+  for (int c = 0; c < VPU; c++)
 #pragma unroll
-    for (int c = 0; c < VPU; c++) {
-      const uint32_t line = llo0 + (uint32_t)(w * (16 / F::WORD) + u * VPU + c);
-      const typename F::Tw* row = a.tw_tab + (size_t)line * 256u + am;
+    for (int i = 0; i < PER; i++) {
+      const int aa = am + L * i;  // outputs b = 0 .. L - 1 are line entries aa + R1 b
+      E y[L];
 #pragma unroll
-      for (int b = 0; b < 16; b++) v[c][b] = F::mul_tw(v[c][b], row[16 * b]);
-    }
-  } else if constexpr (TW) {
+      for (int b = 0; b < L; b++) y[b] = v[c][i * L + b];
+      if constexpr (F::ID == GOLDILOCKS)
+        dft_reg_tw<F, LL, INV>(y, [&](int ll) { return tab1[(ll - 1) * R1 + aa]; });
+      else  // column passes and inverse row passes multiply every result
+        dft_reg<F, LL, INV, TW || INV>(y);
+      const uint32_t line = llo0 + (uint32_t)(ch * (16 / F::WORD) + u * VPU + c) + lm * a.tw_line_mul_m;
+      if (TW && a.tw_tab != nullptr) {
+        // twiddle table [line][k]: one operand per output (tw_line_mul_m == 0)
+        const typename F::Tw* row = a.tw_tab + ((size_t)line << LOGT) + aa;
 #pragma unroll
-    for (int c = 0; c < VPU; c++) {
-      const uint32_t line = llo0 + (uint32_t)(w * (16 / F::WORD) + u * VPU + c) + lm * a.tw_line_mul_m;
-      const uint32_t ls = line * a.tw_scale;
-      const uint32_t e0 = (ls * (uint32_t)am) & a.tw_mask;
-      const uint32_t es = (ls * 16u) & a.tw_mask;
-      E t = F::mul_tw(__ldg(&a.tw_lo[e0 & ((1u << kTwLoBits) - 1)]), a.tw_hi[e0 >> kTwLoBits]);
-      const E step = F::mul_tw(__ldg(&a.tw_lo[es & ((1u << kTwLoBits) - 1)]), a.tw_hi[es >> kTwLoBits]);
+        for (int b = 0; b < L; b++) y[b] = F::mul_tw(y[b], row[R1 * b]);
+      } else if constexpr (TW) {
+        const uint32_t ls = line * a.tw_scale;
+        const uint32_t e0 = (ls * (uint32_t)aa) & a.tw_mask;
+        const uint32_t es = (ls * (uint32_t)R1) & a.tw_mask;
+        E t = F::mul_tw(__ldg(&a.tw_lo[e0 & ((1u << kTwLoBits) - 1)]), a.tw_hi[e0 >> kTwLoBits]);
+        const E step = F::mul_tw(__ldg(&a.tw_lo[es & ((1u << kTwLoBits) - 1)]), a.tw_hi[es >> kTwLoBits]);
 #pragma unroll
-      for (int b = 0; b < 16; b++) {
-        v[c][b] = mul_m<F>(v[c][b], t);
-        if (b + 1 < 16) t = F::mont_mul(t, step);
+        for (int b = 0; b < L; b++) {
+          y[b] = mul_m<F>(y[b], t);
+          if (b + 1 < L) t = F::mont_mul(t, step);
+        }
+      }
+      if constexpr (INV && !TW) {  // the last pass of an inverse transform
+#pragma unroll
+        for (int b = 0; b < L; b++) y[b] = F::mul_tw(y[b], a.scale);
+      }
+#pragma unroll
+      for (int b = 0; b < L; b++) {
+        if constexpr (MODE != MODE_COL) y[b] = F::canon(y[b]);  // the transform's results
+        v[c][i * L + b] = y[b];
       }
     }
-  }
-  if constexpr (INV && !TW) {  // the last pass of an inverse transform
-#pragma unroll
-    for (int c = 0; c < VPU; c++)
-#pragma unroll
-      for (int b = 0; b < 16; b++) v[c][b] = F::mul_tw(v[c][b], a.scale);
-  }
-  if constexpr (MODE != MODE_COL) {  // the transform's results
-#pragma unroll
-    for (int c = 0; c < VPU; c++)
-#pragma unroll
-      for (int b = 0; b < 16; b++) v[c][b] = F::canon(v[c][b]);
-  }
-  if constexpr (ROWS) {
-#pragma unroll
-    for (int b = 0; b < 16; b++) {
-      E x[VPU];
-#pragma unroll
-      for (int c = 0; c < VPU; c++) x[c] = v[c][b];
-      wide_store_unit<F, true>(s, am + 16 * b, w, u, x);
-    }
-  }
+  if constexpr (ROWS) wide_store_rows<F, LOGT>(s, w, v);
 }
 
-template <class F, int MODE, bool INV, bool TW>
+template <class F, int LOGT, int MODE, bool INV, bool TW>
 __global__ void __launch_bounds__(kWideThreads, 3)  // shared memory holds three CTAs an SM
     ntt_wide_pass(const __grid_constant__ CUtensorMap in_map,
                   const __grid_constant__ CUtensorMap out_map, const PassArgs<F> a, int* err) {
   using E = typename F::E;
   using Tw = typename F::Tw;
-  constexpr int C = wide_cols<F>(), VPU = slab_vpu<F>();
-  constexpr int BB = wide_buf_bytes<F>();
+  constexpr int C = wide_cols<F, LOGT>(), VPU = slab_vpu<F>();
+  constexpr int BB = wide_buf_bytes<F, LOGT>();
   extern __shared__ __align__(1024) unsigned char wide_smem_raw[];
   __shared__ __align__(8) uint64_t bars[2];
   __shared__ int abort_flag;
@@ -311,19 +386,16 @@ __global__ void __launch_bounds__(kWideThreads, 3)  // shared memory holds three
     // this one's output): every global access of the pass follows this wait
     grid_dep_wait();
     if (tile < ntiles) {
-      wide_issue_load<F, MODE>(&in_map, a, tile, base, &bars[0]);
+      wide_issue_load<F, LOGT, MODE>(&in_map, a, tile, base, &bars[0]);
       outstanding |= 1u;
     }
     if (tile + gridDim.x < ntiles) {
-      wide_issue_load<F, MODE>(&in_map, a, tile + gridDim.x, base + BB, &bars[1]);
+      wide_issue_load<F, LOGT, MODE>(&in_map, a, tile + gridDim.x, base + BB, &bars[1]);
       outstanding |= 2u;
     }
   }
   grid_dep_launch();
-  for (int i = threadIdx.x; i < 15 * 16; i += kWideThreads) {
-    const int aa = i / 16 + 1, l = i % 16;
-    tab1[i] = a.roots[(uint32_t)(l * aa) * a.roots_stride];  // omega_256^(l a)
-  }
+  wide_fill_tab<F, LOGT>(tab1, a, kWideThreads);
   __syncthreads();
 
   uint32_t phase = 0;
@@ -340,29 +412,22 @@ __global__ void __launch_bounds__(kWideThreads, 3)  // shared memory holds three
     uint32_t g, lm;
     uint64_t lb;
     tile_coords<F, C>(a, tile, g, lm, lb);
-    E v[VPU][16];
-    wide_lines<F, MODE, INV, TW>(a, s, tab1, warp, g * C, lm, v);
+    E v[VPU][1 << wide_r1_log<LOGT>()];
+    wide_lines<F, LOGT, MODE, INV, TW>(a, s, tab1, warp, g * C, lm, v);
     if constexpr (MODE != MODE_COL) {
       // every warp has read its lines: re-lay the results as swizzled rows
       __syncthreads();
-      const int lane = threadIdx.x & 31;
-#pragma unroll
-      for (int bb = 0; bb < 16; bb++) {
-        E x[VPU];
-#pragma unroll
-        for (int c = 0; c < VPU; c++) x[c] = v[c][bb];
-        wide_store_unit<F, true>(s, wide_lane_l(lane) + 16 * bb, warp, wide_lane_u(lane), x);
-      }
+      wide_store_rows<F, LOGT>(s, warp, v);
     }
     fence_proxy_async();  // this thread's writes become visible to the TMA store
     __syncthreads();
     if (abort_flag) break;
     if (threadIdx.x == 0) {
-      wide_issue_store<F, MODE>(&out_map, a, tile, s);
+      wide_issue_store<F, LOGT, MODE>(&out_map, a, tile, s);
       if (tile + 2ull * gridDim.x < ntiles) {
         bulk_wait_read_all();  // the store has read the buffer
         fence_proxy_async();
-        wide_issue_load<F, MODE>(&in_map, a, tile + 2ull * gridDim.x, s, &bars[b]);
+        wide_issue_load<F, LOGT, MODE>(&in_map, a, tile + 2ull * gridDim.x, s, &bars[b]);
         outstanding |= 1u << b;
       }
     }
@@ -408,19 +473,19 @@ constexpr int wide_ws_threads() {
 }
 constexpr int kWideSlots = 6;
 
-template <class F>
+template <class F, int LOGT>
 constexpr size_t wide_ws_smem_bytes() {
-  return kWideSlots * (size_t)wide_buf_bytes<F>() + 15 * 16 * sizeof(typename F::Tw) + 1024;
+  return kWideSlots * (size_t)wide_buf_bytes<F, LOGT>() + wide_tab_entries<F, LOGT>() * sizeof(typename F::Tw) + 1024;
 }
 
-template <class F, int MODE, bool INV, bool TW>
+template <class F, int LOGT, int MODE, bool INV, bool TW>
 __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
     ntt_wide_ws_pass(const __grid_constant__ CUtensorMap in_map,
                      const __grid_constant__ CUtensorMap out_map, const PassArgs<F> a, int* err) {
   using E = typename F::E;
   using Tw = typename F::Tw;
-  constexpr int C = wide_cols<F>(), VPU = slab_vpu<F>(), S = kWideSlots;
-  constexpr int BB = wide_buf_bytes<F>();
+  constexpr int C = wide_cols<F, LOGT>(), VPU = slab_vpu<F>(), S = kWideSlots;
+  constexpr int BB = wide_buf_bytes<F, LOGT>();
   extern __shared__ __align__(1024) unsigned char wide_ws_smem_raw[];
   __shared__ __align__(8) uint64_t full[S], done[S], rd[S], empty[S];
   __shared__ uint32_t unit_next;
@@ -454,7 +519,7 @@ __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
     }
     go = __shfl_sync(0xffffffffu, go, 0);
     if (!go) return false;
-    wide_issue_load_warp<F, MODE>(&in_map, a, tile_of(j_load), base + s * BB, &full[s], lane);
+    wide_issue_load_warp<F, LOGT, MODE>(&in_map, a, tile_of(j_load), base + s * BB, &full[s], lane);
     j_load++;
     return true;
   };
@@ -484,10 +549,7 @@ __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
     }
   }
   grid_dep_launch();
-  for (int i = threadIdx.x; i < 15 * 16; i += wide_ws_threads<F>()) {
-    const int aa = i / 16 + 1, l = i % 16;
-    tab1[i] = a.roots[(uint32_t)(l * aa) * a.roots_stride];  // omega_256^(l a)
-  }
+  wide_fill_tab<F, LOGT>(tab1, a, wide_ws_threads<F>());
   __syncthreads();
 
   if (loader) {
@@ -511,7 +573,7 @@ __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
         abort_flag = 1;
       }
       if (abort_flag) break;
-      wide_issue_store<F, MODE>(&out_map, a, tile_of(j), base + s * BB);
+      wide_issue_store<F, LOGT, MODE>(&out_map, a, tile_of(j), base + s * BB);
       if (j + S < njobs) {
         bulk_wait_read_all();
         mbar_arrive(&empty[s]);
@@ -544,8 +606,8 @@ __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
     uint32_t g, lm;
     uint64_t lb;
     tile_coords<F, C>(a, tile_of(j), g, lm, lb);
-    E v[VPU][16];
-    wide_lines<F, MODE, INV, TW>(a, buf, tab1, w, g * C, lm, v);
+    E v[VPU][1 << wide_r1_log<LOGT>()];
+    wide_lines<F, LOGT, MODE, INV, TW>(a, buf, tab1, w, g * C, lm, v);
     if constexpr (MODE != MODE_COL) {
       // the rows of the output span every column group's lines: re-lay after
       // all eight units have read theirs
@@ -558,13 +620,7 @@ __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
         }
         break;
       }
-#pragma unroll
-      for (int bb = 0; bb < 16; bb++) {
-        E x[VPU];
-#pragma unroll
-        for (int c = 0; c < VPU; c++) x[c] = v[c][bb];
-        wide_store_unit<F, true>(buf, wide_lane_l(lane) + 16 * bb, w, wide_lane_u(lane), x);
-      }
+      wide_store_rows<F, LOGT>(buf, w, v);
     }
     fence_proxy_async();  // this thread's writes become visible to the TMA store
     __syncwarp();

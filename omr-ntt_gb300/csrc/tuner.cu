@@ -9,7 +9,8 @@
 //     every plan of the count-point transform, and every full plan followed
 //     by a gather.
 // omr_ntt_tune_point times every candidate on device buffers it owns (CUDA
-// events, L2 flushed before each timed run, median of `reps`); the caller
+// events, L2 flushed before each timed run of one or more calls, median of
+// `reps`); the caller
 // records the fastest in the planner database (omr_ntt_planner_*), which the
 // planner (plan = -1) consults before its built-in heuristic.  All candidates
 // are exact, so the choice changes speed, never a result.
@@ -506,16 +507,23 @@ int omr_ntt_tune_point(int field, uint32_t log_n, uint64_t batch, int pattern, u
     // warm-up (also builds sub-domains and scratch outside the timed runs)
     rc = run_candidate(d, cands[i], pattern, count, idx, in, out, batch, st);
     if (rc) break;
+    // a timed run is one call, or for short candidates as many back to back
+    // as make about 0.2 ms: event times come in steps of 2 us on GB300
     std::vector<float> t;
-    for (int r = 0; r < reps && !rc; r++) {
+    int calls = 1;
+    for (int r = -1; r < reps && !rc; r++) {
       cudaMemsetAsync(flush, r & 0xff, flush_bytes, st);
       cudaEventRecord(e0, st);
-      rc = run_candidate(d, cands[i], pattern, count, idx, in, out, batch, st);
+      for (int k = 0; k < calls && !rc; k++)
+        rc = run_candidate(d, cands[i], pattern, count, idx, in, out, batch, st);
       cudaEventRecord(e1, st);
       if (cudaEventSynchronize(e1) != cudaSuccess) rc = fail(OMR_NTT_ERR_CUDA, "tuning sync");
       float ms = 0;
       cudaEventElapsedTime(&ms, e0, e1);
-      t.push_back(ms);
+      if (r < 0)
+        calls = std::max(1, std::min(24, (int)(0.2f / std::max(ms, 1e-3f))));
+      else
+        t.push_back(ms / (float)calls);
     }
     std::sort(t.begin(), t.end());
     if (i < cap && ms_out) ms_out[i] = t.empty() ? -1.f : t[t.size() / 2];
