@@ -196,8 +196,8 @@ const std::vector<PlanShape>& plan_table(uint32_t log_n) {
   return log_n <= 32 ? table[log_n] : none;
 }
 
-std::vector<PassDesc> build_passes(uint32_t log_n, uint64_t batch, const PlanShape& shape) {
-  std::vector<PassDesc> ps;
+PassList build_passes(uint32_t log_n, uint64_t batch, const PlanShape& shape) {
+  PassList ps;
   const uint64_t N = 1ull << log_n;
   const int P = (int)shape.split.size();
   auto base = [&](int logT) {
@@ -406,7 +406,7 @@ int run_transform(omr_ntt_domain_s* d, int plan, bool inverse, const void* in, v
     if (in != out) OMR_CUDA_TRY(cudaMemcpyAsync(out, in, bytes, cudaMemcpyDeviceToDevice, stream));
     return OMR_NTT_OK;
   }
-  std::vector<PassDesc> ps = build_passes(d->log_n, batch, d->plans[plan]);
+  const PassList ps = build_passes(d->log_n, batch, d->plans[plan]);
   if (d->plans[plan].variant == kClusterVariant) {
     int rc = launch_cluster_transform(d, ps, inverse, in, out, batch, stream);
     if (rc <= 0) return rc;  // launched, or an error; 1: run the passes below
@@ -531,10 +531,7 @@ int omr_ntt_domain_create(int field, uint32_t log_n, omr_ntt_domain_t* out) {
     return fail(OMR_NTT_ERR_ALLOC, "error-word allocation failed");
   }
   int rc = with_field(field, [&](auto f) { return build_domain_tables<decltype(f)>(d); });
-  if (rc == OMR_NTT_OK) {
-    RootTables rt;
-    rc = get_root_tables(field, &rt);
-  }
+  if (rc == OMR_NTT_OK) rc = get_root_tables(field, &d->roots);
   if (rc) {
     omr_ntt_domain_destroy(d);
     return rc;
@@ -692,8 +689,7 @@ int omr_ntt_plan_passes(int field, uint32_t log_n, int plan, uint64_t batch, uin
   if (cnt < 0) return cnt;
   if (plan < 0) plan = default_plan(field, log_n, batch);
   if (plan >= cnt) return fail(OMR_NTT_ERR_INVALID_ARGUMENT, "plan id out of range");
-  std::vector<PassDesc> ps =
-      log_n ? build_passes(log_n, batch, plan_table(log_n)[plan]) : std::vector<PassDesc>{};
+  const PassList ps = log_n ? build_passes(log_n, batch, plan_table(log_n)[plan]) : PassList{};
   for (int i = 0; i < (int)ps.size() && i < cap && rec; i++) {
     const PassDesc& p = ps[i];
     uint64_t* r = rec + 16 * i;
@@ -723,7 +719,7 @@ int omr_ntt_plan_run_pass(omr_ntt_domain_t d, int plan, int pass, int inverse, c
   if (plan < 0) plan = default_plan(d->field, d->log_n, batch);
   if (plan >= (int)d->plans.size()) return fail(OMR_NTT_ERR_INVALID_ARGUMENT, "plan id out of range");
   if (batch == 0 || d->log_n == 0) return OMR_NTT_OK;
-  std::vector<PassDesc> ps = build_passes(d->log_n, batch, d->plans[plan]);
+  const PassList ps = build_passes(d->log_n, batch, d->plans[plan]);
   if (pass < 0 || pass >= (int)ps.size()) return fail(OMR_NTT_ERR_INVALID_ARGUMENT, "pass out of range");
   const PassDesc& p = ps[pass];
   if ((p.in_buf == 1 || p.out_buf == 1) && !scratch)

@@ -79,7 +79,15 @@ struct PlanShape {
 std::vector<PlanShape> enumerate_plans(uint32_t log_n);
 // enumerate_plans(log_n) for log_n <= 32, built once (no allocation per call)
 const std::vector<PlanShape>& plan_table(uint32_t log_n);
-std::vector<PassDesc> build_passes(uint32_t log_n, uint64_t batch, const PlanShape& shape);
+// The passes of a plan (at most three; no allocation).
+struct PassList {
+  PassDesc p[3];
+  int n = 0;
+  size_t size() const { return (size_t)n; }
+  const PassDesc& operator[](size_t i) const { return p[i]; }
+  void push_back(const PassDesc& d) { p[n++] = d; }
+};
+PassList build_passes(uint32_t log_n, uint64_t batch, const PlanShape& shape);
 int default_plan(int field, uint32_t log_n, uint64_t batch);
 // The planner's full-transform plan: planner database, learned selector, else
 // built-in heuristic (tuner.cu).  use_learned = false skips the learned
@@ -87,7 +95,7 @@ int default_plan(int field, uint32_t log_n, uint64_t batch);
 int planned_full_plan(int field, uint32_t log_n, uint64_t batch, bool use_learned = true);
 // One-launch transform of a two-pass plan on an 8-CTA cluster (ntt_cluster.cu):
 // 0 launched, 1 not available for this shape (run the passes), < 0 error.
-int launch_cluster_transform(const omr_ntt_domain_s* d, const std::vector<PassDesc>& ps,
+int launch_cluster_transform(const omr_ntt_domain_s* d, const PassList& ps,
                              bool inverse, const void* in, void* out, uint64_t batch,
                              cudaStream_t stream);
 constexpr int kClusterVariant = 3;  // PlanShape::variant of the cluster plans
@@ -133,6 +141,7 @@ struct omr_ntt_domain_s {
   void* tw_hi_f = nullptr;
   void* tw_lo_i = nullptr;
   void* tw_hi_i = nullptr;
+  omr::RootTables roots;  // the field's in-line root tables on this device
   int* err = nullptr;  // device error word raised by bounded waits (OMR_NTT_ERR_TIMEOUT)
   std::mutex mu;       // guards `scratch`
   std::mutex host_mu;  // serialises the synchronous host-buffer calls

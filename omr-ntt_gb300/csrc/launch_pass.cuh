@@ -569,9 +569,7 @@ int make_pass_args(const omr_ntt_domain_s* d, const PassDesc& p, bool inverse, c
                    void* out, bool last, PassArgs<F>* out_args) {
   using E = typename F::E;
   using Tw = typename F::Tw;
-  RootTables rt;
-  int rc = get_root_tables(F::ID, &rt);
-  if (rc) return rc;
+  const RootTables& rt = d->roots;
   PassArgs<F>& a = *out_args;
   a = PassArgs<F>{};
   a.in = static_cast<const E*>(in);

@@ -85,7 +85,7 @@ extern "C" int omr_ntt_forward_noalloc(omr_ntt_domain_t d, const void* in, void*
     return OMR_NTT_OK;
   }
   const int plan = planned_full_plan(d->field, d->log_n, batch, /*use_learned=*/false);
-  const std::vector<PassDesc> ps = build_passes(d->log_n, batch, d->plans[plan]);
+  const PassList ps = build_passes(d->log_n, batch, d->plans[plan]);
   if (d->plans[plan].variant == kClusterVariant) {
     // the one-launch cluster plan keeps its intermediate in shared memory
     int rc = launch_cluster_transform(d, ps, false, in, out, batch, st);

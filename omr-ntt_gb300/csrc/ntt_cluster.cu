@@ -156,7 +156,7 @@ static int launch_cluster_dir(int log1, int log2, const PassArgs<F>& a, const Pa
 
 // 0: launched; 1: this shape has no cluster kernel or could not be launched
 // (the caller then runs the plan's passes); < 0: error.
-int launch_cluster_transform(const omr_ntt_domain_s* d, const std::vector<PassDesc>& ps,
+int launch_cluster_transform(const omr_ntt_domain_s* d, const PassList& ps,
                              bool inverse, const void* in, void* out, uint64_t batch,
                              cudaStream_t stream) {
   if (ps.size() != 2) return 1;

@@ -256,9 +256,7 @@ inline int launch_prefix_t(omr_ntt_domain_s* d, uint32_t m, const uint32_t* idx,
     occ_cache[dev & 63] = occ < 1 ? 1 : occ;
     occ = occ_cache[dev & 63];
   }
-  RootTables rt;
-  int rc = get_root_tables(F::ID, &rt);
-  if (rc) return rc;
+  const RootTables& rt = d->roots;
   PassArgs<F> a{};
   a.in = static_cast<const E*>(in);
   a.L_lo = (uint32_t)(d->n >> LOGT);  // columns r
@@ -277,7 +275,7 @@ inline int launch_prefix_t(omr_ntt_domain_s* d, uint32_t m, const uint32_t* idx,
   uint32_t grid = (uint32_t)device_sm_count(dev) * (uint32_t)occ;
   if (grid > groups) grid = groups;
   void* part = nullptr;
-  rc = domain_scratch(d, stream, (size_t)grid * m * sizeof(E), &part, 1);
+  const int rc = domain_scratch(d, stream, (size_t)grid * m * sizeof(E), &part, 1);
   if (rc) return rc;
   OMR_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(NT), smem, stream, a, m, idx, static_cast<E*>(part)));
   return launch_reduce_rows<F>(static_cast<const E*>(part), grid, m, static_cast<E*>(out), stream);

@@ -19,7 +19,7 @@ import ctypes
 import numpy as np
 
 from . import _lib
-from ._lib import OmrNttError, check, lib
+from ._lib import OmrNttError, check, current_raw_stream, lib
 from .fields import BabyBear, DefaultField, Field, Goldilocks, KoalaBear, TeddyBear, field_by_id
 from .inputs import gen_input_seeded, random_indices
 from . import encoders
@@ -39,13 +39,11 @@ def _is_tensor(x) -> bool:
 
 
 def _stream_of(x, stream):
+    """The stream handle (an int) of a call on `x`: the caller's, else torch's
+    current stream of a CUDA tensor's device, else the default stream."""
     if stream is not None:
-        return ctypes.c_void_p(int(stream))
-    if _is_tensor(x):
-        import torch
-
-        return ctypes.c_void_p(torch.cuda.current_stream(x.device).cuda_stream)
-    return ctypes.c_void_p(0)
+        return int(stream)
+    return current_raw_stream(x) if _is_tensor(x) else 0
 
 
 class NttDomain:
@@ -124,8 +122,7 @@ def _transform(domain, x, plan, out, batch, stream, inverse):
     if _is_tensor(x):
         dst = x if out is None else out
         fn = L.omr_ntt_inverse if inverse else L.omr_ntt_forward
-        check(fn(domain.handle, plan, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(dst.data_ptr()),
-                 batch, _stream_of(x, stream)))
+        check(fn(domain.handle, plan, x.data_ptr(), dst.data_ptr(), batch, _stream_of(x, stream)))
         return dst
     a = _host_array(domain.field, x).copy()
     fn = L.omr_ntt_inverse_host if inverse else L.omr_ntt_forward_host
@@ -138,13 +135,13 @@ def partial(domain: NttDomain, x, pattern: int, count: int, indices=None, out=No
     X[j N/count] (STRIDED) or X[indices] (INDICES)."""
     L = lib()
     if _is_tensor(x):
-        import torch
-
         if out is None:
+            import torch
+
             out = torch.empty(count, dtype=x.dtype, device=x.device)
-        idx_ptr = ctypes.c_void_p(indices.data_ptr()) if indices is not None else None
-        check(L.omr_ntt_partial(domain.handle, pattern, count, idx_ptr, ctypes.c_void_p(x.data_ptr()),
-                                ctypes.c_void_p(out.data_ptr()), _stream_of(x, stream)))
+        idx_ptr = indices.data_ptr() if indices is not None else None
+        check(L.omr_ntt_partial(domain.handle, pattern, count, idx_ptr, x.data_ptr(), out.data_ptr(),
+                                _stream_of(x, stream)))
         return out
     a = _host_array(domain.field, x)
     res = np.empty(count, dtype=domain.field.dtype)

@@ -136,6 +136,23 @@ def lib():
     return _lib
 
 
+_raw_stream = None
+
+
+def current_raw_stream(x) -> int:
+    """Handle of torch's current stream on the device of CUDA tensor `x`.  The
+    handle itself costs 0.1 us; torch.cuda.current_stream builds a Stream
+    object around it (2 us, a quarter of a small transform's call)."""
+    global _raw_stream
+    import torch
+
+    if _raw_stream is None:
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", False)
+    if _raw_stream and x.is_cuda:
+        return _raw_stream(x.get_device())
+    return torch.cuda.current_stream(x.device).cuda_stream
+
+
 def declared_symbols():
     return list(_SIGS)
 

@@ -10,9 +10,7 @@ src/encoders/tfhe_stockham_radix8.rs:17-21).
 """
 from __future__ import annotations
 
-import ctypes
-
-from ._lib import check, lib
+from ._lib import check, current_raw_stream, lib
 
 ARK_RADIX2, DFT, DFT_PARTIAL, LAMBDA_BOWERS, LAMBDA_RADIX4 = 0, 1, 2, 3, 4
 PLONKY3_LAYER_SPLIT, TFHE_STOCKHAM_R8, TRANSFORM_DECOMPOSITION = 5, 6, 7
@@ -29,11 +27,8 @@ class NttEncoder:
         """In-place forward NTT of ``buf`` (NumPy array or CUDA tensor)."""
         L = lib()
         if hasattr(buf, "data_ptr") and hasattr(buf, "is_cuda"):
-            import torch
-
-            st = stream if stream is not None else torch.cuda.current_stream(buf.device).cuda_stream
-            check(L.omr_ntt_encode(domain.handle, self.ID, self.s, ctypes.c_void_p(buf.data_ptr()),
-                                   batch, ctypes.c_void_p(int(st))))
+            st = int(stream) if stream is not None else current_raw_stream(buf)
+            check(L.omr_ntt_encode(domain.handle, self.ID, self.s, buf.data_ptr(), batch, st))
             return buf
         if not buf.flags["C_CONTIGUOUS"] or buf.dtype != domain.field.dtype:
             raise TypeError("buf must be a C-contiguous array of the field's word type")
