@@ -183,6 +183,9 @@ std::vector<PlanShape> enumerate_plans(uint32_t log_n) {
   for (auto& s : splits)
     if (s.size() > 1 && std::all_of(s.begin(), s.end(), [](int t) { return t == 8; }))
       out.push_back(PlanShape{s, kTcVariant});
+  // 2^10..2^12: the balanced two-pass plan as one cluster launch (appended)
+  if (log_n >= 10 && log_n <= 12)
+    out.push_back(PlanShape{{(int)(log_n + 1) / 2, (int)log_n / 2}, kClusterVariant});
   return out;
 }
 

@@ -278,10 +278,27 @@ enum { DST_SMEM = 0, DST_GLOBAL = 1, DST_STAGE = 2 };  // STAGE: smem tile, four
 // mapping: 8 lines x 4 rows per warp, one sector per row); DST_GLOBAL writes
 // the output directly (c-fast, or j-fast for MODE_LINE so a warp writes 32
 // consecutive words of one line).
+// Four-step twiddle of one butterfly group (line, outputs k = d + q NS): base
+// omega_N^(line d scale) and step omega_N^(line NS scale).
+template <class F>
+struct TwPair {
+  typename F::E cur, step;
+};
+template <class F>
+OMR_D TwPair<F> group_twiddle(const PassArgs<F>& a, uint32_t line, uint32_t d, uint32_t ns) {
+  const uint32_t ls = line * a.tw_scale;
+  const uint32_t eb = (ls * d) & a.tw_mask, es = (ls * ns) & a.tw_mask;
+  return {F::mul_tw(a.tw_lo[eb & ((1u << kTwLoBits) - 1)], a.tw_hi[eb >> kTwLoBits]),
+          F::mul_tw(a.tw_lo[es & ((1u << kTwLoBits) - 1)], a.tw_hi[es >> kTwLoBits])};
+}
+
+// `pre` (DST_STAGE only): the round's group twiddles where the caller has
+// them already, one per group of the thread.
 template <class F, int LOGT, int C, int NT, int LOGR, int LOGNS, bool INV, int SRC, int DST,
           bool JF, bool TW>
 OMR_D void do_round(const PassArgs<F>& a, typename F::E* s, const typename F::E* __restrict__ gin,
-                    typename F::E* __restrict__ gout, int nvalid, uint32_t llo0, uint32_t lm) {
+                    typename F::E* __restrict__ gout, int nvalid, uint32_t llo0, uint32_t lm,
+                    const TwPair<F>* pre = nullptr) {
   using E = typename F::E;
   constexpr int T = 1 << LOGT, R = 1 << LOGR, NS = 1 << LOGNS;
   constexpr int TR = T / R;
@@ -329,10 +346,9 @@ OMR_D void do_round(const PassArgs<F>& a, typename F::E* s, const typename F::E*
       if constexpr (TW && DST != DST_SMEM) {
         has_tw = (DST == DST_STAGE || a.tw_lo != nullptr) && c < nvalid;
         if (has_tw) {
-          const uint32_t ls = (llo0 + (uint32_t)c + lm * a.tw_line_mul_m) * a.tw_scale;
-          const uint32_t eb = (ls * (uint32_t)d) & a.tw_mask, es = (ls * (uint32_t)NS) & a.tw_mask;
-          tw_cur = F::mul_tw(a.tw_lo[eb & ((1u << kTwLoBits) - 1)], a.tw_hi[eb >> kTwLoBits]);
-          tw_step = F::mul_tw(a.tw_lo[es & ((1u << kTwLoBits) - 1)], a.tw_hi[es >> kTwLoBits]);
+          const TwPair<F> t = pre ? pre[i] : group_twiddle(a, llo0 + (uint32_t)c + lm * a.tw_line_mul_m, (uint32_t)d, NS);
+          tw_cur = t.cur;
+          tw_step = t.step;
         }
       }
 #pragma unroll

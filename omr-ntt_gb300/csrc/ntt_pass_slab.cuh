@@ -344,7 +344,6 @@ template <class F, int LOGT, int MODE, bool INV, bool TW>
 __global__ void __launch_bounds__(slab_threads<LOGT>(), (slab_min_blocks<F, LOGT>()))
     ntt_slab_pass(const __grid_constant__ CUtensorMap in_map,
                   const __grid_constant__ CUtensorMap out_map, const PassArgs<F> a, int* err) {
-  pdl_entry();
   using Tw = typename F::Tw;
   constexpr int R0 = 1 << slab_r0_log<LOGT>(), C = slab_cols<F>();
   constexpr int NT = slab_threads<LOGT>();
@@ -368,14 +367,10 @@ __global__ void __launch_bounds__(slab_threads<LOGT>(), (slab_min_blocks<F, LOGT
     fence_proxy_async();
     abort_flag = 0;
   }
-  __syncthreads();
-  bool outstanding = false;  // this warp's load into its slab has not been waited for
-  if (leader && tile < ntiles) {
-    slab_issue_load<F, LOGT, MODE>(&in_map, a, tile, warp, my_slab, &bar);
-    outstanding = true;
-  }
   // in-line twiddle tables: tab0[(k1 - 1) 256 + j] = omega_T^(j k1),
-  // tab1[(a - 1) 16 + l] = omega_256^(l a) = omega_T^(l a R0)
+  // tab1[(a - 1) 16 + l] = omega_256^(l a) = omega_T^(l a R0); filled before
+  // the wait on the previous kernel (its output is this pass's input), so
+  // that their lookups overlap its tail
   for (int i = threadIdx.x; i < (R0 - 1) * 256; i += NT) {
     const int k1 = i / 256 + 1, j = i % 256;
     tab0[i] = a.roots[(uint32_t)(j * k1) * a.roots_stride];
@@ -385,6 +380,12 @@ __global__ void __launch_bounds__(slab_threads<LOGT>(), (slab_min_blocks<F, LOGT
     tab1[i] = a.roots[(uint32_t)(l * aa * R0) * a.roots_stride];
   }
   __syncthreads();
+  pdl_entry();
+  bool outstanding = false;  // this warp's load into its slab has not been waited for
+  if (leader && tile < ntiles) {
+    slab_issue_load<F, LOGT, MODE>(&in_map, a, tile, warp, my_slab, &bar);
+    outstanding = true;
+  }
 
   uint32_t phase = 0;
   for (; tile < ntiles; tile += gridDim.x) {

@@ -386,7 +386,6 @@ template <class F, int LOGT, int C, int NT, int MODE, bool INV, bool TW, int NBU
 __global__ void __launch_bounds__(NT, (tma_min_blocks<F, LOGT, NT, NBUF>()))
     ntt_tile_pass_tma(const __grid_constant__ CUtensorMap in_map,
                       const __grid_constant__ CUtensorMap out_map, const PassArgs<F> a, int* err) {
-  pdl_entry();
   using E = typename F::E;
   using Tw = typename F::Tw;
   constexpr size_t BW = tma_buf_words<F, LOGT, C>();
@@ -411,7 +410,11 @@ __global__ void __launch_bounds__(NT, (tma_min_blocks<F, LOGT, NT, NBUF>()))
     fence_proxy_async();
     abort_flag = 0;
   }
+  // the tables before the wait on the previous kernel (its output is this
+  // pass's input), so that their lookups overlap its tail
+  build_rtw<F, LOGT, 1>(srtw, a.roots, a.roots_stride, NT);
   __syncthreads();
+  pdl_entry();
   uint64_t tile = blockIdx.x;
   bool outstanding[2] = {false, false};  // a load into the buffer has not been waited for
   if (threadIdx.x == 0) {
@@ -424,9 +427,7 @@ __global__ void __launch_bounds__(NT, (tma_min_blocks<F, LOGT, NT, NBUF>()))
       outstanding[1] = true;
     }
   }
-  build_rtw<F, LOGT, 1>(srtw, a.roots, a.roots_stride, NT);
   const SmemTw<F> st{srtw, a.tw_lo, a.tw_hi};
-  // (the first loop iteration's barrier publishes the staged tables)
 
   uint32_t phase = 0;
   int it = 0;

@@ -71,7 +71,7 @@ static std::vector<Cand> candidates(int field, uint32_t log_n, int pattern, uint
 //           kind 0: balanced split with the fewest passes, 1: its reverse,
 //           2: balanced with one more pass, 3: large-first (4096, ..., 4096, remainder);
 //           class 3 itself (plain tile pass, large-first: never the fastest
-//           on GB300) stands for the one-launch cluster plan of 2^13..2^16
+//           on GB300) stands for the one-launch cluster plan of 2^10..2^16
 //   20..23  decomposition (prefix or index set) with line length next_pow2(count) << j, j = 0..3
 //   24..43  strided fold, then the count-point transform with full class (c - 24)
 //   44..63  full transform with full class (c - 44), then gather

@@ -1,6 +1,7 @@
 """GPU parity of the passes that are chosen by the number of tiles, on both
 sides of each line: the two-round pass at 512- and 1024-point lines and the
-wide pass at 64- and 128-point lines, forward and inverse, against the oracle.
+wide pass at 64- and 128-point lines; and the cluster plans of the smallest
+sizes.  Forward and inverse, against the oracle.
 Half of each input is words at the ends of the canonical range."""
 import numpy as np
 import pytest
@@ -27,6 +28,9 @@ CASES = [
     # Goldilocks: column passes from 2048 tiles, plain row passes
     (Goldilocks, 20, 4, "64x128x128 slab"), (Goldilocks, 20, 8, "64x128x128 slab"), (Goldilocks, 20, 9, "128x128x64 slab"),
     (Goldilocks, 22, 1, "256x128x128 wide"),
+    # one cluster a transform, the smallest sizes in odd batches
+    (BabyBear, 10, 3, "32x32 cluster"), (Goldilocks, 10, 1, "32x32 cluster"), (KoalaBear, 11, 5, "64x32 cluster"),
+    (TeddyBear, 12, 7, "64x64 cluster"), (Goldilocks, 12, 9, "64x64 cluster"),
 ]
 
 
