@@ -227,13 +227,21 @@ OMR_D void slab_round0(unsigned char* buf, const typename F::Tw* tab0) {
   }
 }
 
+template <class F, int MODE>
+OMR_D int slab_lane_l(int lane) {  // (see slab_rounds12)
+  return MODE == MODE_COL || F::WORD == 4 ? ((lane & 7) | ((lane >> 1) & 8)) : (lane & 15);
+}
+template <class F, int MODE>
+OMR_D int slab_lane_u(int lane) {
+  return MODE == MODE_COL || F::WORD == 4 ? ((lane >> 3) & 1) : (lane >> 4);
+}
 // Rounds 1 and 2 of one warp on its slab; the results end in the slab as
 // interleaved [a + 16 b][column] rows (the store layout).
 template <class F, int LOGT, int MODE, bool INV, bool TW>
 OMR_D void slab_rounds12(const PassArgs<F>& a, unsigned char* s, const typename F::Tw* tab1,
-                         int k1, uint32_t llo0, uint32_t lm) {
+                         const TwPair<F> (&chain)[slab_vpu<F>()]) {
   using E = typename F::E;
-  constexpr int R0 = 1 << slab_r0_log<LOGT>(), VPU = slab_vpu<F>();
+  constexpr int VPU = slab_vpu<F>();
   const int lane = threadIdx.x & 31;
   // 16-byte rows (r * 16 + 8 u: column passes, and every pass's final
   // staging) take 8-byte accesses a half-warp at a time, so each half-warp
@@ -243,9 +251,7 @@ OMR_D void slab_rounds12(const PassArgs<F>& a, unsigned char* s, const typename 
   // line-major rounds of row passes are conflict-free with it for 4-byte
   // words; for 8-byte (Goldilocks) words there l = lane & 15, u = lane >> 4
   // is, so those row passes keep that assignment.
-  constexpr bool kHalfWarp = MODE == MODE_COL || F::WORD == 4;
-  const int l = kHalfWarp ? ((lane & 7) | ((lane >> 1) & 8)) : (lane & 15);
-  const int u = kHalfWarp ? ((lane >> 3) & 1) : (lane >> 4);
+  const int l = slab_lane_l<F, MODE>(lane), u = slab_lane_u<F, MODE>(lane);
   E v[VPU][16];
   // round 1: lane l transforms rows l + 16 m (m < 16) of its column unit
 #pragma unroll
@@ -298,12 +304,8 @@ OMR_D void slab_rounds12(const PassArgs<F>& a, unsigned char* s, const typename 
   if constexpr (TW) {
 #pragma unroll
     for (int c = 0; c < VPU; c++) {
-      const uint32_t line = llo0 + (uint32_t)(u * VPU + c) + lm * a.tw_line_mul_m;
-      const uint32_t ls = line * a.tw_scale;
-      const uint32_t e0 = (ls * (uint32_t)(k1 + R0 * am)) & a.tw_mask;
-      const uint32_t es = (ls * (uint32_t)(16 * R0)) & a.tw_mask;
-      E w = F::mul_tw(__ldg(&a.tw_lo[e0 & ((1u << kTwLoBits) - 1)]), a.tw_hi[e0 >> kTwLoBits]);
-      const E step = F::mul_tw(__ldg(&a.tw_lo[es & ((1u << kTwLoBits) - 1)]), a.tw_hi[es >> kTwLoBits]);
+      E w = chain[c].cur;
+      const E step = chain[c].step;
 #pragma unroll
       for (int b = 0; b < 16; b++) {
         v[c][b] = mul_m<F>(v[c][b], w);
@@ -389,6 +391,21 @@ __global__ void __launch_bounds__(slab_threads<LOGT>(), (slab_min_blocks<F, LOGT
 
   uint32_t phase = 0;
   for (; tile < ntiles; tile += gridDim.x) {
+    uint32_t g, lm;
+    uint64_t lb;
+    tile_coords<F, C>(a, tile, g, lm, lb);
+    // the four-step chains of the lane's lines, looked up before the wait for
+    // the tile's data, whose latency covers theirs
+    TwPair<F> chain[slab_vpu<F>()];
+    if constexpr (TW) {
+      const int lane = threadIdx.x & 31;
+#pragma unroll
+      for (int c = 0; c < slab_vpu<F>(); c++)
+        chain[c] = group_twiddle(a,
+                                 g * C + (uint32_t)(slab_lane_u<F, MODE>(lane) * slab_vpu<F>() + c) +
+                                     lm * a.tw_line_mul_m,
+                                 (uint32_t)(warp + R0 * slab_lane_l<F, MODE>(lane)), 16u * R0);
+    }
     // every thread waits for the tile's slabs (bounded); a timeout raises the
     // error word and the flag, read by all after the barrier below
     if (mbar_wait_bounded(&bar, phase)) {
@@ -398,13 +415,10 @@ __global__ void __launch_bounds__(slab_threads<LOGT>(), (slab_min_blocks<F, LOGT
       atomicExch(err, OMR_NTT_ERR_TIMEOUT);
       abort_flag = 1;
     }
-    uint32_t g, lm;
-    uint64_t lb;
-    tile_coords<F, C>(a, tile, g, lm, lb);
     if constexpr (R0 > 1) slab_round0<F, LOGT, MODE, INV>(buf, tab0);
     __syncthreads();  // every slab complete (and the waits' verdicts published)
     if (abort_flag) break;
-    slab_rounds12<F, LOGT, MODE, INV, TW>(a, my_slab, tab1, warp, g * C, lm);
+    slab_rounds12<F, LOGT, MODE, INV, TW>(a, my_slab, tab1, chain);
     fence_proxy_async();  // this lane's slab writes become visible to the TMA store
     __syncwarp();
     if (leader) {
