@@ -69,8 +69,8 @@ struct BatchArgs {
   char* out;
   char* scratch;
   const uint32_t* idx;
-  const void* roots_bb;  // omega_4096 tables (forward)
-  const void* roots_gl;
+  const void* rtw_bb;  // in-line twiddle tables (forward)
+  const void* rtw_gl;
 };
 
 template <class F>
@@ -128,8 +128,7 @@ OMR_D void batch_col_tile(const BatchArgs& ba, const BatchReq& r, uint32_t g, ty
   a.L_lo = n2;
   a.es_in = n2;
   a.es_out = n2;
-  a.roots = static_cast<const Tw*>(F::ID == BABYBEAR ? ba.roots_bb : ba.roots_gl);
-  a.roots_stride = 1u << (kMaxLogT - LOGT);
+  a.rtw = static_cast<const Tw*>(F::ID == BABYBEAR ? ba.rtw_bb : ba.rtw_gl);
   a.tw_lo = static_cast<const E*>(r.tw_lo);
   a.tw_hi = static_cast<const Tw*>(r.tw_hi);
   a.tw_scale = 1;
@@ -180,8 +179,7 @@ OMR_D void batch_row_tile(const BatchArgs& ba, const BatchReq& r, uint32_t g, ty
   }
   __syncthreads();
   PassArgs<F> a{};
-  a.roots = static_cast<const Tw*>(F::ID == BABYBEAR ? ba.roots_bb : ba.roots_gl);
-  a.roots_stride = 1u << (kMaxLogT - LOGT);
+  a.rtw = static_cast<const Tw*>(F::ID == BABYBEAR ? ba.rtw_bb : ba.rtw_gl);
   batch_row_rounds<F, LOGT, C, 0>(a, s, nvalid, llo0);
   E* dst = reinterpret_cast<E*>(r.partial ? ba.scratch + r.scr_b : ba.out + r.out_off);
   const typename F::Tw scale = F::make_tw(r.n_inv);
@@ -379,8 +377,8 @@ static BatchArgs batch_args(omr_ntt_batch_s* b, const void* in, void* out) {
   a.out = static_cast<char*>(out);
   a.scratch = b->d_scratch;
   a.idx = b->d_idx;
-  a.roots_bb = bb.fwd;
-  a.roots_gl = gl.fwd;
+  a.rtw_bb = bb.fwd;
+  a.rtw_gl = gl.fwd;
   return a;
 }
 

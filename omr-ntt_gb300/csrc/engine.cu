@@ -68,7 +68,7 @@ static int build_root_tables(RootTables* out) {
   const uint64_t w = root_of_unity_host<F>(kMaxLogT);
   const uint64_t wi = hpowmod(w, p - 2, p);
   const int T = 1 << kMaxLogT;
-  std::vector<Tw> f(T), iv(T);
+  std::vector<Tw> f(T), iv(T);  // omega_4096^k
   uint64_t a = 1, b = 1;
   for (int k = 0; k < T; k++) {
     f[k] = F::make_tw(a);
@@ -76,11 +76,22 @@ static int build_root_tables(RootTables* out) {
     a = hmulmod(a, w, p);
     b = hmulmod(b, wi, p);
   }
+  std::vector<Tw> rf(kRoundTableWords), ri(kRoundTableWords);  // every round shape's [q][jm] (ntt_pass.cuh)
+  for (int lr = 1; lr <= kMaxTableRadixLog; lr++)
+    for (int lns = 0; lr + lns <= kMaxLogT; lns++)
+      for (int q = 0; q < 1 << lr; q++)
+        for (int jm = 0; jm < 1 << lns; jm++) {
+          const size_t at = round_table_off(lr, lns) + ((size_t)q << lns) + jm;
+          const size_t e = ((size_t)q * jm) << (kMaxLogT - lr - lns);
+          rf[at] = f[e];
+          ri[at] = iv[e];
+        }
   void *df = nullptr, *di = nullptr;
-  OMR_CUDA_TRY(cudaMalloc(&df, sizeof(Tw) * T));
-  OMR_CUDA_TRY(cudaMalloc(&di, sizeof(Tw) * T));
-  OMR_CUDA_TRY(cudaMemcpy(df, f.data(), sizeof(Tw) * T, cudaMemcpyHostToDevice));
-  OMR_CUDA_TRY(cudaMemcpy(di, iv.data(), sizeof(Tw) * T, cudaMemcpyHostToDevice));
+  const size_t bytes = sizeof(Tw) * kRoundTableWords;
+  OMR_CUDA_TRY(cudaMalloc(&df, bytes));
+  OMR_CUDA_TRY(cudaMalloc(&di, bytes));
+  OMR_CUDA_TRY(cudaMemcpy(df, rf.data(), bytes, cudaMemcpyHostToDevice));
+  OMR_CUDA_TRY(cudaMemcpy(di, ri.data(), bytes, cudaMemcpyHostToDevice));
   out->fwd = df;
   out->inv = di;
   return OMR_NTT_OK;

@@ -113,8 +113,8 @@ int planned_partial(int field, uint32_t log_n, int pattern, uint64_t count, int*
                     int* param);
 
 // ------------------------------------------------------------------ device tables
-// Per-field in-line roots omega_4096^k, k < 4096 (forward and inverse),
-// stored as F::Tw, built once per device.
+// Per-field in-line twiddles of every round shape (round_table, ntt_pass.cuh;
+// forward and inverse), stored as F::Tw, built once per device.
 struct RootTables {
   const void* fwd = nullptr;
   const void* inv = nullptr;

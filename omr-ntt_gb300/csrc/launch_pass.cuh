@@ -584,8 +584,7 @@ int make_pass_args(const omr_ntt_domain_s* d, const PassDesc& p, bool inverse, c
   a.os_b = p.os_b;
   a.es_in = (uint32_t)p.es_in;
   a.es_out = (uint32_t)p.es_out;
-  a.roots = static_cast<const Tw*>(inverse ? rt.inv : rt.fwd);
-  a.roots_stride = (uint32_t)(1u << (kMaxLogT - p.logT));
+  a.rtw = static_cast<const Tw*>(inverse ? rt.inv : rt.fwd);
   if (p.twiddle) {
     a.tw_lo = static_cast<const E*>(inverse ? d->tw_lo_i : d->tw_lo_f);
     a.tw_hi = static_cast<const Tw*>(inverse ? d->tw_hi_i : d->tw_hi_f);

@@ -46,20 +46,20 @@ constexpr int cluster_threads(int log_n) {
 
 template <class F, int LOG1, int W, int NT, bool INV, int I>
 OMR_D void cluster_columns(const PassArgs<F>& a, typename F::E* s, const typename F::E* gin,
-                           uint32_t llo0, const TwPair<F>* pre) {
+                           uint32_t llo0, const TwPair<F>* pre, const typename F::Tw* staged) {
   using RP = RoundPlan<LOG1, max_radix_log<F>()>;
   if constexpr (I < RP::ROUNDS) {
     constexpr int SRC = I == 0 ? SRC_GLOBAL : SRC_SMEM;
     constexpr int DST = I + 1 == RP::ROUNDS ? DST_STAGE : DST_SMEM;
     do_round<F, LOG1, W, NT, RP::logr(I), RP::logns(I), INV, SRC, DST, false, true>(a, s, gin, nullptr, W, llo0, 0,
-                                                                                   pre);
-    cluster_columns<F, LOG1, W, NT, INV, I + 1>(a, s, gin, llo0, pre);
+                                                                                   pre, staged);
+    cluster_columns<F, LOG1, W, NT, INV, I + 1>(a, s, gin, llo0, pre, staged);
   }
 }
 
 template <class F, int LOG1, int LOG2, bool INV>
 __global__ void __launch_bounds__(cluster_threads(LOG1 + LOG2))
-    ntt_cluster_kernel(const PassArgs<F> ga, const PassArgs<F> gb) {
+    ntt_cluster_kernel(const PassArgs<F> a, const PassArgs<F> b) {
   using E = typename F::E;
   using Tw = typename F::Tw;
   constexpr int CL = cluster_ctas(LOG1 + LOG2), NT = cluster_threads(LOG1 + LOG2);
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(cluster_threads(LOG1 + LOG2))
   constexpr int W = N2 / CL;  // pass-1 columns per CTA
   constexpr int H = N1 / CL;  // pass-2 rows per CTA
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ Tw roots[N1];                 // omega_N1^k; omega_N2^k at stride N1 / N2
+  __shared__ Tw rt1[N1], rt2[N2];          // in-line twiddles (each line has one twiddled round)
   E* ta = reinterpret_cast<E*>(smem_raw);  // [N1][W], tile_idx<F, W>
   E* tb = ta + N1 * W;                     // [N2][H], tile_idx<F, H>
   cg::cluster_group cluster = cg::this_cluster();
@@ -75,13 +75,12 @@ __global__ void __launch_bounds__(cluster_threads(LOG1 + LOG2))
   const uint64_t t = blockIdx.x / CL;  // transform of the batch
 
   // tables only: nothing here depends on the previous kernel
-  PassArgs<F> a = ga, b = gb;
-  for (int i = threadIdx.x; i < N1; i += NT) roots[i] = a.roots[(uint32_t)i * a.roots_stride];
-  a.roots = b.roots = roots;
-  a.roots_stride = 1;
-  b.roots_stride = N1 / N2;
   using RP = RoundPlan<LOG1, max_radix_log<F>()>;
-  constexpr int LR = RP::logr(RP::ROUNDS - 1), LNS = RP::logns(RP::ROUNDS - 1);
+  using RP2 = RoundPlan<LOG2, max_radix_log<F>()>;
+  static_assert(RP::ROUNDS == 2 && RP2::ROUNDS == 2, "one twiddled round a line");
+  constexpr int LR = RP::logr(1), LNS = RP::logns(1);
+  for (int i = threadIdx.x; i < N1; i += NT) rt1[i] = round_table<F, LR, LNS>(a)[i];
+  for (int i = threadIdx.x; i < N2; i += NT) rt2[i] = round_table<F, RP2::logr(1), RP2::logns(1)>(b)[i];
   constexpr int NB = (N1 >> LR) * W, PER = (NB + NT - 1) / NT;  // groups of the last column round (do_round)
   TwPair<F> pre[PER];
 #pragma unroll
@@ -96,7 +95,7 @@ __global__ void __launch_bounds__(cluster_threads(LOG1 + LOG2))
   __syncthreads();
   pdl_entry();
 
-  cluster_columns<F, LOG1, W, NT, INV, 0>(a, ta, a.in + t * a.is_b + r * W, r * W, pre);
+  cluster_columns<F, LOG1, W, NT, INV, 0>(a, ta, a.in + t * a.is_b + r * W, r * W, pre, rt1);
   cluster.sync();  // every pass-1 tile complete and visible to the cluster
 
   // all of a thread's remote loads are issued before its local stores: the
@@ -118,7 +117,7 @@ __global__ void __launch_bounds__(cluster_threads(LOG1 + LOG2))
     tb[tile_idx<F, H>(idx % N2, idx / N2)] = g[k];
   }
   __syncthreads();
-  all_rounds<F, LOG2, H, NT, MODE_ROW, INV, 0>(b, tb, nullptr, b.out + t * b.os_b + r * H, H, 0, 0);
+  all_rounds<F, LOG2, H, NT, MODE_ROW, INV, 0>(b, tb, nullptr, b.out + t * b.os_b + r * H, H, 0, 0, rt2);
   cluster.sync();  // no CTA exits while a peer may still read its tile
 }
 

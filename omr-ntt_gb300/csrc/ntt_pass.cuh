@@ -66,9 +66,8 @@ struct PassArgs {
   uint64_t is_lo, is_m, is_b;  // input strides of the line index components
   uint64_t os_lo, os_m, os_b;  // output strides
   uint32_t es_in, es_out;      // element strides along a line (within a transform: < 2^31)
-  // in-line roots: roots[k * roots_stride] = omega_T^k (forward or inverse)
-  const Tw* roots;
-  uint32_t roots_stride;
+  // in-line twiddles of every round shape (round_table)
+  const Tw* rtw;
   // four-step twiddle on outputs: exponent e = (tw_line * k * tw_scale) mod N,
   // tw_line = llo + lm * tw_line_mul_m; tw_lo == nullptr disables it
   const E* tw_lo;   // omega^i (i < 2^12), "twiddle-Montgomery" form
@@ -83,6 +82,22 @@ struct PassArgs {
   // chain with one table operand per output
   const Tw* tw_tab;
 };
+
+// In-line twiddles.  A Stockham round of radix R on subtransforms of NS points
+// multiplies input q of a group by omega_{NS R}^(q jm), jm < NS: a table of
+// [q][jm] that depends on R and NS only.  All of them (R = 2 .. 32, NS R <=
+// 4096) lie in one array per field and direction, so that the lanes of a warp,
+// which hold neighbouring jm, read neighbouring words -- the same operands
+// gathered from one table of omega_4096 powers touch up to 32 lines an access.
+constexpr int kMaxTableRadixLog = 5;
+constexpr size_t kRoundTableWords = (size_t)kMaxTableRadixLog << (kMaxLogT + 1);
+constexpr size_t round_table_off(int logr, int logns) {
+  return ((size_t)(logr - 1) << (kMaxLogT + 1)) + ((size_t)1 << (logr + logns));
+}
+template <class F, int LOGR, int LOGNS>
+OMR_D const typename F::Tw* round_table(const PassArgs<F>& a) {
+  return a.rtw + round_table_off(LOGR, LOGNS);
+}
 
 // --------------------------------------------------------------- helpers
 template <class F>
@@ -293,12 +308,13 @@ OMR_D TwPair<F> group_twiddle(const PassArgs<F>& a, uint32_t line, uint32_t d, u
 }
 
 // `pre` (DST_STAGE only): the round's group twiddles where the caller has
-// them already, one per group of the thread.
+// them already, one per group of the thread.  `staged`: the round's in-line
+// twiddles where the caller has staged them (round_table's layout).
 template <class F, int LOGT, int C, int NT, int LOGR, int LOGNS, bool INV, int SRC, int DST,
           bool JF, bool TW>
 OMR_D void do_round(const PassArgs<F>& a, typename F::E* s, const typename F::E* __restrict__ gin,
                     typename F::E* __restrict__ gout, int nvalid, uint32_t llo0, uint32_t lm,
-                    const TwPair<F>* pre = nullptr) {
+                    const TwPair<F>* pre = nullptr, const typename F::Tw* staged = nullptr) {
   using E = typename F::E;
   constexpr int T = 1 << LOGT, R = 1 << LOGR, NS = 1 << LOGNS;
   constexpr int TR = T / R;
@@ -331,9 +347,8 @@ OMR_D void do_round(const PassArgs<F>& a, typename F::E* s, const typename F::E*
       const int j = JF ? b % TR : b / C;
       const int jm = j & (NS - 1);
       if constexpr (LOGNS > 0) {
-        // a_q *= omega_{NS*R}^{q*jm} = omega_T^{q*jm*T/(NS*R)}
-        constexpr int SCALE = T / (NS * R);
-        dft_reg_tw<F, LOGR, INV>(v[i], [&](int q) { return a.roots[(uint32_t)(q * jm * SCALE) * a.roots_stride]; });
+        const typename F::Tw* tw = (staged ? staged : round_table<F, LOGR, LOGNS>(a)) + jm;
+        dft_reg_tw<F, LOGR, INV>(v[i], [&](int q) { return tw[q * NS]; });
       } else {
         dft_reg<F, LOGR, INV>(v[i]);
       }
@@ -391,7 +406,8 @@ OMR_D void do_round(const PassArgs<F>& a, typename F::E* s, const typename F::E*
 
 template <class F, int LOGT, int C, int NT, int MODE, bool INV, int I>
 OMR_D void all_rounds(const PassArgs<F>& a, typename F::E* s, const typename F::E* gin,
-                      typename F::E* gout, int nvalid, uint32_t llo0, uint32_t lm) {
+                      typename F::E* gout, int nvalid, uint32_t llo0, uint32_t lm,
+                      const typename F::Tw* staged = nullptr) {
   using RP = RoundPlan<LOGT, max_radix_log<F>()>;
   if constexpr (I < RP::ROUNDS) {
     constexpr bool first = I == 0, last = I + 1 == RP::ROUNDS;
@@ -399,9 +415,9 @@ OMR_D void all_rounds(const PassArgs<F>& a, typename F::E* s, const typename F::
     constexpr int DST = last ? DST_GLOBAL : DST_SMEM;
     constexpr bool JF = last && MODE == MODE_LINE;
     constexpr bool TW = MODE == MODE_COL;
-    do_round<F, LOGT, C, NT, RP::logr(I), RP::logns(I), INV, SRC, DST, JF, TW>(a, s, gin, gout,
-                                                                              nvalid, llo0, lm);
-    all_rounds<F, LOGT, C, NT, MODE, INV, I + 1>(a, s, gin, gout, nvalid, llo0, lm);
+    do_round<F, LOGT, C, NT, RP::logr(I), RP::logns(I), INV, SRC, DST, JF, TW>(
+        a, s, gin, gout, nvalid, llo0, lm, nullptr, staged);
+    all_rounds<F, LOGT, C, NT, MODE, INV, I + 1>(a, s, gin, gout, nvalid, llo0, lm, staged);
   }
 }
 

@@ -241,10 +241,7 @@ __global__ void __launch_bounds__(duo_teams<LOGT>() * duo_team_threads<LOGT>(),
     for (uint32_t j = 0; j < (uint32_t)NB && j < njobs; j++) issue(j);
   }
   grid_dep_launch();
-  for (int i = threadIdx.x; i < 31 * L; i += TEAMS * NT) {
-    const int aa = i / L + 1, l = i % L;
-    tab[i] = a.roots[(uint32_t)(l * aa) * a.roots_stride];
-  }
+  for (int i = threadIdx.x; i < 31 * L; i += TEAMS * NT) tab[i] = round_table<F, 5, LOGT - 5>(a)[L + i];
   __syncthreads();
 
   const int team = TEAMS == 1 ? 0 : (int)(threadIdx.x / NT);

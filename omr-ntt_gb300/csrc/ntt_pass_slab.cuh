@@ -373,14 +373,9 @@ __global__ void __launch_bounds__(slab_threads<LOGT>(), (slab_min_blocks<F, LOGT
   // tab1[(a - 1) 16 + l] = omega_256^(l a) = omega_T^(l a R0); filled before
   // the wait on the previous kernel (its output is this pass's input), so
   // that their lookups overlap its tail
-  for (int i = threadIdx.x; i < (R0 - 1) * 256; i += NT) {
-    const int k1 = i / 256 + 1, j = i % 256;
-    tab0[i] = a.roots[(uint32_t)(j * k1) * a.roots_stride];
-  }
-  for (int i = threadIdx.x; i < 15 * 16; i += NT) {
-    const int aa = i / 16 + 1, l = i % 16;
-    tab1[i] = a.roots[(uint32_t)(l * aa * R0) * a.roots_stride];
-  }
+  if constexpr (R0 > 1)
+    for (int i = threadIdx.x; i < (R0 - 1) * 256; i += NT) tab0[i] = round_table<F, slab_r0_log<LOGT>(), 8>(a)[256 + i];
+  for (int i = threadIdx.x; i < 15 * 16; i += NT) tab1[i] = round_table<F, 4, 4>(a)[16 + i];
   __syncthreads();
   pdl_entry();
   bool outstanding = false;  // this warp's load into its slab has not been waited for

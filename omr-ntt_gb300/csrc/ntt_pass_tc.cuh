@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     reinterpret_cast<uint4*>(sB)[i] = reinterpret_cast<const uint4*>(bmat)[i];
   for (int i = threadIdx.x; i < 15 * 16; i += kTcThreads) {
     const int aa = i / 16 + 1, l = i % 16;
-    tab1[i] = a.roots[(uint32_t)(l * aa) * a.roots_stride];  // omega_256^(l a)
+    tab1[i] = round_table<F, 4, 4>(a)[16 * aa + l];  // omega_256^(l a)
   }
   fence_proxy_async();  // B is read by the tensor cores (async proxy)
   __syncthreads();

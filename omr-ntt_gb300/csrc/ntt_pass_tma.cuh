@@ -167,18 +167,15 @@ constexpr size_t tma_smem_total() {
 }
 
 template <class F, int LOGT, int RI>
-OMR_D void build_rtw(typename F::Tw* dst, const typename F::Tw* __restrict__ roots,
-                     uint32_t roots_stride, int nt) {
+OMR_D void build_rtw(typename F::Tw* dst, const PassArgs<F>& a, int nt) {
   using RP = RoundPlan<LOGT, max_radix_log<F>()>;
   if constexpr (RI < RP::ROUNDS) {
     if constexpr (RI >= 1) {
       constexpr int R = 1 << RP::logr(RI), NS = 1 << RP::logns(RI);
-      constexpr int SCALE = (1 << LOGT) / (NS * R);
       constexpr int OFF = rtw_off<LOGT, max_radix_log<F>()>(RI);
-      for (int k = threadIdx.x; k < R * NS; k += nt)
-        dst[OFF + k] = roots[(uint32_t)((k / NS) * (k % NS) * SCALE) * roots_stride];
+      for (int k = threadIdx.x; k < R * NS; k += nt) dst[OFF + k] = round_table<F, RP::logr(RI), RP::logns(RI)>(a)[k];
     }
-    build_rtw<F, LOGT, RI + 1>(dst, roots, roots_stride, nt);
+    build_rtw<F, LOGT, RI + 1>(dst, a, nt);
   }
 }
 
@@ -412,7 +409,7 @@ __global__ void __launch_bounds__(NT, (tma_min_blocks<F, LOGT, NT, NBUF>()))
   }
   // the tables before the wait on the previous kernel (its output is this
   // pass's input), so that their lookups overlap its tail
-  build_rtw<F, LOGT, 1>(srtw, a.roots, a.roots_stride, NT);
+  build_rtw<F, LOGT, 1>(srtw, a, NT);
   __syncthreads();
   pdl_entry();
   uint64_t tile = blockIdx.x;

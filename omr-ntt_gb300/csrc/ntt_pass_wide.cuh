@@ -96,9 +96,10 @@ constexpr size_t wide_smem_bytes() {
 template <class F, int LOGT>
 OMR_D void wide_fill_tab(typename F::Tw* tab1, const PassArgs<F>& a, int nt) {
   constexpr int R1 = 1 << wide_r1_log<LOGT>(), L = (1 << LOGT) / R1;
-  constexpr int W = F::ID == GOLDILOCKS ? R1 : L;  // table width
+  constexpr int LW = F::ID == GOLDILOCKS ? wide_r1_log<LOGT>() : LOGT - wide_r1_log<LOGT>();  // log2 table width
+  static_assert(wide_tab_entries<F, LOGT>() == (F::ID == GOLDILOCKS ? (L - 1) * R1 : (R1 - 1) * L), "whole rows");
   for (int i = threadIdx.x; i < wide_tab_entries<F, LOGT>(); i += nt)
-    tab1[i] = a.roots[(uint32_t)((i / W + 1) * (i % W)) * a.roots_stride];
+    tab1[i] = round_table<F, LOGT - LW, LW>(a)[(1 << LW) + i];
 }
 
 // 128-byte-swizzled row layout: byte of (row r, 16-byte chunk ch, offset o)

@@ -264,8 +264,7 @@ inline int launch_prefix_t(omr_ntt_domain_s* d, uint32_t m, const uint32_t* idx,
   a.L_b = 1;
   a.is_lo = 1;
   a.es_in = (uint32_t)(d->n >> LOGT);
-  a.roots = static_cast<const Tw*>(rt.fwd);
-  a.roots_stride = 1u << (kMaxLogT - LOGT);
+  a.rtw = static_cast<const Tw*>(rt.fwd);
   a.tw_lo = static_cast<const E*>(d->tw_lo_f);
   a.tw_hi = static_cast<const Tw*>(d->tw_hi_f);
   a.tw_scale = 1;
