@@ -73,10 +73,16 @@ struct BatchArgs {
   const void* rtw_gl;
 };
 
+// Lines per tile: 8192 (BabyBear) or 4096 (Goldilocks) words a tile, so that a
+// radix-16 round has one or two butterflies for each of the 256 threads (with
+// 2048 words, half of them idled in the rounds of 256-point lines), at least
+// 32 bytes of lines, and no more lines than the smallest request of the line
+// length has (32 lines of 32 points, 64 of 64).
 template <class F>
 constexpr int batch_cols(int logt) {
-  int c = 2048 >> logt;
-  if (c > 64) c = 64;
+  const int cap = logt == 5 ? 32 : 64;
+  int c = (F::WORD == 8 ? 4096 : 8192) >> logt;
+  if (c > cap) c = cap;
   return c < 32 / F::WORD ? 32 / F::WORD : c;
 }
 
@@ -86,17 +92,15 @@ OMR_D unsigned int ld_acquire(const unsigned int* p) {
   return v;
 }
 
-// The persistent kernel runs every line length of both fields in one body
-// with a tight register budget: Goldilocks keeps radix-8 rounds there.
-template <class F>
-constexpr int batch_radix_log() {
-  return F::WORD == 8 ? 3 : 4;
-}
+// Radix of the rounds.  Goldilocks radix-16 rounds spill in the 64 registers
+// of the kernel, and still beat radix 8 (mixed 4096 requests 8.6 against 9.1
+// ms on GB300): a round and its exchange less at 256 and 1024 points.
+constexpr int kBatchRadixLog = 4;
 
 template <class F, int LOGT, int C, int I>
 OMR_D void batch_col_rounds(const PassArgs<F>& a, typename F::E* s, const typename F::E* gin,
                             typename F::E* gout, int nvalid, uint32_t llo0) {
-  using RP = RoundPlan<LOGT, batch_radix_log<F>()>;
+  using RP = RoundPlan<LOGT, kBatchRadixLog>;
   if constexpr (I < RP::ROUNDS) {
     constexpr bool first = I == 0, last = I + 1 == RP::ROUNDS;
     do_round<F, LOGT, C, kBatchThreads, RP::logr(I), RP::logns(I), false,
@@ -108,7 +112,7 @@ OMR_D void batch_col_rounds(const PassArgs<F>& a, typename F::E* s, const typena
 
 template <class F, int LOGT, int C, int I>
 OMR_D void batch_row_rounds(const PassArgs<F>& a, typename F::E* s, int nvalid, uint32_t llo0) {
-  using RP = RoundPlan<LOGT, batch_radix_log<F>()>;
+  using RP = RoundPlan<LOGT, kBatchRadixLog>;
   if constexpr (I < RP::ROUNDS) {
     constexpr bool last = I + 1 == RP::ROUNDS;
     do_round<F, LOGT, C, kBatchThreads, RP::logr(I), RP::logns(I), false, SRC_SMEM,
@@ -240,10 +244,11 @@ OMR_D void batch_dispatch(const BatchArgs& ba, const BatchReq& r, const BatchTas
 // so the claim's round trip overlaps the current tile.  A CTA still runs its
 // tickets in increasing order, so the smallest unfinished task is always some
 // CTA's current task with every dependency done: the queue cannot deadlock.
-// Three CTAs per SM (<= 80 registers, a few hundred bytes of spills): the
-// tasks are short and latency bound, and the extra resident CTA measured
-// 12% faster on the 4096-request workload than two CTAs at 128 registers.
-__global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(const BatchArgs ba) {
+// Four CTAs per SM (<= 64 registers): the tasks are short and latency bound
+// (a claim, a dependency wait, the loads, the rounds and the stores in turn),
+// and what hides one CTA's latencies is the others.  4096 requests on GB300:
+// 8.5 ms; 9.2 with three CTAs at 80 registers, 10.4 with five at 48.
+__global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(const BatchArgs ba) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t task_id;
   __shared__ int abort_flag;
