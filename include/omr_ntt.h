@@ -254,7 +254,8 @@ int omr_ntt_batch_info(omr_ntt_batch_t b, uint64_t *requests, uint64_t *tasks,
                        uint64_t *scratch_bytes);
 
 /* Run the whole batch: one graph launch (counter reset + persistent kernel).
- * The graph is re-captured when the arena pointers change. */
+ * The graph is captured on the first run; other arena pointers become new
+ * arguments of its kernel node. */
 int omr_ntt_batch_run(omr_ntt_batch_t b, const void *in, void *out, void *stream);
 
 /* Synchronise and report a bounded dependency wait that gave up. */

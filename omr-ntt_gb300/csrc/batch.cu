@@ -328,6 +328,7 @@ struct omr_ntt_batch_s {
   // graph
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  cudaGraphNode_t kernel_node = nullptr;
   const void* g_in = nullptr;
   void* g_out = nullptr;
   int grid = 0;
@@ -365,6 +366,22 @@ static void batch_free_device(omr_ntt_batch_s* b) {
   b->d_ctr = nullptr;
   b->d_err = nullptr;
   b->d_scratch = nullptr;
+}
+
+// The kernel node of the captured graph (memset, kernel).
+static cudaError_t batch_kernel_node(omr_ntt_batch_s* b) {
+  cudaGraphNode_t nodes[4];
+  size_t n = 4;
+  cudaError_t e = cudaGraphGetNodes(b->graph, nodes, &n);
+  for (size_t i = 0; e == cudaSuccess && i < n; i++) {
+    cudaGraphNodeType t;
+    e = cudaGraphNodeGetType(nodes[i], &t);
+    if (e == cudaSuccess && t == cudaGraphNodeTypeKernel) {
+      b->kernel_node = nodes[i];
+      return cudaSuccess;
+    }
+  }
+  return e == cudaSuccess ? cudaErrorInvalidValue : e;
 }
 
 static BatchArgs batch_args(omr_ntt_batch_s* b, const void* in, void* out) {
@@ -539,11 +556,7 @@ int omr_ntt_batch_run(omr_ntt_batch_t b, const void* in, void* out, void* stream
   }
   DeviceGuard g(b->device);
   cudaStream_t st = (cudaStream_t)stream;
-  if (!b->exec || b->g_in != in || b->g_out != out) {
-    if (b->exec) cudaGraphExecDestroy(b->exec);
-    if (b->graph) cudaGraphDestroy(b->graph);
-    b->exec = nullptr;
-    b->graph = nullptr;
+  if (!b->exec) {
     cudaStream_t cap = nullptr;
     OMR_CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
     const BatchArgs a = batch_args(b, in, out);
@@ -553,9 +566,29 @@ int omr_ntt_batch_run(omr_ntt_batch_t b, const void* in, void* out, void* stream
       batch_kernel<<<b->grid, kBatchThreads, kBatchSmem, cap>>>(a);
       e = cudaStreamEndCapture(cap, &b->graph);
     }
+    if (e == cudaSuccess) e = batch_kernel_node(b);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec, b->graph, 0);
     cudaStreamDestroy(cap);
-    if (e != cudaSuccess) return fail(OMR_NTT_ERR_CUDA, std::string("batch graph: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+      if (b->graph) cudaGraphDestroy(b->graph);
+      b->graph = nullptr;
+      b->exec = nullptr;
+      return fail(OMR_NTT_ERR_CUDA, std::string("batch graph: ") + cudaGetErrorString(e));
+    }
+    b->g_in = in;
+    b->g_out = out;
+  } else if (b->g_in != in || b->g_out != out) {
+    // other arenas: new arguments for the kernel node (runs already launched
+    // keep theirs)
+    BatchArgs a = batch_args(b, in, out);
+    void* args[] = {&a};
+    cudaKernelNodeParams kp = {};
+    kp.func = (void*)batch_kernel;
+    kp.gridDim = dim3((unsigned)b->grid);
+    kp.blockDim = dim3(kBatchThreads);
+    kp.sharedMemBytes = (unsigned)kBatchSmem;
+    kp.kernelParams = args;
+    OMR_CUDA_TRY(cudaGraphExecKernelNodeSetParams(b->exec, b->kernel_node, &kp));
     b->g_in = in;
     b->g_out = out;
   }
