@@ -7,6 +7,7 @@
 
 #include <atomic>
 
+#include "launch_pass.cuh"
 #include "partial.cuh"
 
 namespace omr {
@@ -185,6 +186,132 @@ __global__ void __launch_bounds__(prefix_threads<F, LOGT>(), 2)
   }
 }
 
+// The same sum on the wide pass's tiles, for T = 64, 128 and 256: TMA lands
+// [T rows x 128-byte column boxes] in two buffers, a warp transforms the lines
+// of its 16-byte column groups in registers (wide_lines, ntt_pass_wide.cuh) and
+// leaves Y[k][column] as swizzled rows, and the Horner threads read a row four
+// (two) columns at a time: 47 instead of 69 instructions per input word of the
+// kernel above, which addresses every word of its tile by itself, and smaller
+// tiles.  On GB300, both kernels of 100 BabyBear outputs with T = 128 (256): N =
+// 2^18 7.2 (6.7) us against 11.7 (10.8), 2^22 14.5 (13.5) against 16.6 (15.7),
+// 2^24 35.3 (33.9) against 54.3 (50.5); Goldilocks 2^22 29.3 (27.9) against
+// 32.1 (29.9).
+// Thread (output q, slice): acc = acc omega_N^(-j) + Y[j mod T][r] over the
+// slice's run of columns, times omega_N^(-j (C - run)) between tiles, and
+// omega_N^(j r_last) at the end.
+template <class F, int LOGT>
+constexpr size_t prefix_wide_smem_bytes() {
+  return 2 * (size_t)wide_buf_bytes<F, LOGT>() + wide_tab_entries<F, LOGT>() * sizeof(typename F::Tw) + 1024;
+}
+
+template <class F, int LOGT>
+__global__ void __launch_bounds__(kWideThreads, 3)
+    prefix_wide_kernel(const __grid_constant__ CUtensorMap in_map, const PassArgs<F> a, uint32_t m,
+                       const uint32_t* __restrict__ idx, typename F::E* __restrict__ partial, int* err) {
+  using E = typename F::E;
+  using Tw = typename F::Tw;
+  constexpr int T = 1 << LOGT, C = wide_cols<F, LOGT>(), NCH = 8 * wide_boxes<LOGT>(), VC = 16 / F::WORD;
+  constexpr int BB = wide_buf_bytes<F, LOGT>();
+  extern __shared__ __align__(1024) unsigned char prefix_wide_smem_raw[];
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ int abort_flag;
+  unsigned char* base = prefix_wide_smem_raw + ((1024u - (smem_u32(prefix_wide_smem_raw) & 1023u)) & 1023u);
+  Tw* tab1 = reinterpret_cast<Tw*>(base + 2 * BB);
+  const int warp = threadIdx.x >> 5;
+
+  const uint32_t groups = a.L_lo / C;
+  const uint32_t g0 = (uint32_t)((uint64_t)blockIdx.x * groups / gridDim.x);
+  const uint32_t g1 = (uint32_t)((uint64_t)(blockIdx.x + 1) * groups / gridDim.x);
+  uint32_t outstanding = 0;  // (thread 0) bit b: a load into buffer b has not been waited for
+  if (threadIdx.x == 0) {
+    prefetch_tmap(&in_map);
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+    fence_mbar_init();
+    fence_proxy_async();
+    abort_flag = 0;
+    grid_dep_wait();  // (the input, and the scratch rows a previous call's reduction reads)
+    for (uint32_t b = 0; b < 2 && g0 + b < g1; b++) {
+      wide_issue_load<F, LOGT, MODE_COL>(&in_map, a, g0 + b, base + b * BB, &bars[b]);
+      outstanding |= 1u << b;
+    }
+  }
+  grid_dep_launch();
+  wide_fill_tab<F, LOGT>(tab1, a, kWideThreads);
+
+  // thread -> output slot x column slice
+  uint32_t kact = 1;
+  while (kact < m) kact <<= 1;
+  const uint32_t slices = min((uint32_t)kWideThreads / kact, (uint32_t)NCH), run = NCH / slices;  // run: chunks
+  const uint32_t q = threadIdx.x % kact, slice = threadIdx.x / kact;
+  const bool active = slice < slices && q < m;
+  if (idx != nullptr) grid_dep_wait();
+  const uint32_t j = active ? (idx ? idx[q] : q) : 0u;
+  const bool in_range = (uint64_t)j <= (uint64_t)a.tw_mask;  // an index past N yields 0
+  const int row = (int)(j & (uint32_t)(T - 1));
+  const Tw z1 = omega_tw<F>(a, (uint64_t)0 - (uint64_t)j);
+  const Tw z2 = omega_tw<F>(a, (uint64_t)0 - (uint64_t)(C - run * VC) * j);
+  __syncthreads();
+
+  E acc = 0;
+  uint32_t phase = 0;
+  bool first = true;
+  for (uint32_t g = g0; g < g1; g++) {
+    const uint32_t b = (g - g0) & 1;
+    unsigned char* s = base + b * BB;
+    if (mbar_wait_bounded(&bars[b], (phase >> b) & 1)) {
+      phase ^= 1u << b;
+      outstanding &= ~(1u << b);
+    } else {
+      atomicExch(err, OMR_NTT_ERR_TIMEOUT);
+      abort_flag = 1;
+    }
+    {
+      E v[slab_vpu<F>()][1 << wide_r1_log<LOGT>()];
+      wide_lines<F, LOGT, MODE_COL, false, false>(a, s, tab1, warp, 0, 0, v);
+    }
+    __syncthreads();  // every line's results in the tile
+    if (abort_flag) break;
+    if (active) {
+      if (!first) acc = F::mul_tw(acc, z2);
+#pragma unroll 4
+      for (uint32_t i = 0; i < run; i++) {
+        const uint4 w = *reinterpret_cast<const uint4*>(s + wide_sw<LOGT>(row, (int)(slice * run + i), 0));
+        const E* y = reinterpret_cast<const E*>(&w);
+#pragma unroll
+        for (int c = 0; c < VC; c++) acc = F::mul_add(acc, z1, y[c]);
+      }
+    }
+    first = false;
+    __syncthreads();  // the rows have been read
+    if (threadIdx.x == 0 && g + 2 < g1) {
+      fence_proxy_async();
+      wide_issue_load<F, LOGT, MODE_COL>(&in_map, a, g + 2, s, &bars[b]);
+      outstanding |= 1u << b;
+    }
+  }
+  if (threadIdx.x == 0)
+    for (int b = 0; b < 2; b++)
+      if ((outstanding >> b) & 1) mbar_wait_bounded(&bars[b], (phase >> b) & 1);
+  __syncthreads();
+  if (active) {
+    const uint64_t r_last = (uint64_t)(g1 - 1) * C + (uint64_t)(slice + 1) * run * VC - 1;
+    acc = in_range ? F::canon(mul_m<F>(acc, omega_m<F>(a, r_last * j))) : (E)0;
+  }
+  if (slices > 1) {
+    E* red = reinterpret_cast<E*>(base);
+    if (slice < slices) red[slice * kact + q] = active ? acc : (E)0;
+    __syncthreads();
+    if (threadIdx.x < m) {
+      E sum = 0;
+      for (uint32_t sl = 0; sl < slices; sl++) sum = F::add(sum, red[sl * kact + threadIdx.x]);
+      partial[(uint64_t)blockIdx.x * m + threadIdx.x] = sum;
+    }
+  } else if (threadIdx.x < m) {
+    partial[(uint64_t)blockIdx.x * m + threadIdx.x] = acc;
+  }
+}
+
 // out[k] = sum over rows of partial[row * cols + k].  A CTA of kReduceThreads
 // covers cw adjacent columns (cw a power of two <= 32) with kReduceThreads / cw
 // row slices, so each thread sums only rows / slices values (independent
@@ -236,6 +363,36 @@ inline int launch_reduce_rows(const typename F::E* partial, uint64_t rows, uint6
 }
 
 template <class F, int LOGT>
+inline int launch_prefix_wide(omr_ntt_domain_s* d, PassArgs<F> a, uint32_t m, const uint32_t* idx, int dev,
+                              void* out, cudaStream_t stream) {
+  using E = typename F::E;
+  constexpr int C = wide_cols<F, LOGT>(), T = 1 << LOGT;
+  constexpr size_t smem = prefix_wide_smem_bytes<F, LOGT>();
+  auto kern = prefix_wide_kernel<F, LOGT>;
+  static std::atomic<int> occ_cache[64];
+  int occ = occ_cache[dev & 63].load();
+  if (occ == 0) {
+    OMR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    OMR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kWideThreads, smem));
+    occ_cache[dev & 63] = occ < 1 ? 1 : occ;
+    occ = occ_cache[dev & 63];
+  }
+  CUtensorMap map;
+  if (encode_2d(&map, F::WORD, a.in, a.L_lo, T, a.L_lo, C / wide_boxes<LOGT>(), T, CU_TENSOR_MAP_SWIZZLE_128B) !=
+      CUDA_SUCCESS)
+    return fail(OMR_NTT_ERR_CUDA, "cuTensorMapEncodeTiled (decomposition) failed");
+  const uint32_t groups = a.L_lo / C;
+  uint32_t grid = (uint32_t)device_sm_count(dev) * (uint32_t)occ;
+  if (grid > groups) grid = groups;
+  void* part = nullptr;
+  const int rc = domain_scratch(d, stream, (size_t)grid * m * sizeof(E), &part, 1);
+  if (rc) return rc;
+  OMR_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(kWideThreads), smem, stream, map, a, m, idx,
+                          static_cast<E*>(part), d->err));
+  return launch_reduce_rows<F>(static_cast<const E*>(part), grid, m, static_cast<E*>(out), stream);
+}
+
+template <class F, int LOGT>
 inline int launch_prefix_t(omr_ntt_domain_s* d, uint32_t m, const uint32_t* idx, const void* in,
                            void* out, cudaStream_t stream) {
   using E = typename F::E;
@@ -270,6 +427,10 @@ inline int launch_prefix_t(omr_ntt_domain_s* d, uint32_t m, const uint32_t* idx,
   a.tw_scale = 1;
   a.tw_mask = (uint32_t)(d->n - 1);
   a.tw_line_mul_m = 0;
+  // whole tiles of columns and TMA's alignment: the wide form
+  if constexpr (LOGT >= 6 && LOGT <= 8)
+    if (a.L_lo % wide_cols<F, LOGT>() == 0 && !(reinterpret_cast<uintptr_t>(in) & 15))
+      return launch_prefix_wide<F, LOGT>(d, a, m, idx, dev, out, stream);
   const uint32_t groups = (a.L_lo + C - 1) / C;
   uint32_t grid = (uint32_t)device_sm_count(dev) * (uint32_t)occ;
   if (grid > groups) grid = groups;
