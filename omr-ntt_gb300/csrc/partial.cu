@@ -255,14 +255,19 @@ int partial_dispatch(omr_ntt_domain_s* d, int pattern, uint64_t count, const uin
     return run_strategy_t<F>(d, strategy, param, pattern, count, indices, in, out, stream);
   // built-in rule (timings of the exhaustive tuner on GB300): the fold for
   // strided sets unless they keep more than 2^16 outputs of at most 8 cosets
-  // (then the full transform + gather); the pruned decomposition for <= 4096
-  // outputs of transforms above 2^20, where it beats the full transform
+  // (then the full transform + gather); the pruned decomposition where it
+  // beats the full transform: for <= 256 outputs from 2^16 (2^18, 100 outputs:
+  // 6.7 us against 9.4), for <= 4096 above 2^20.  Lines of 64 points for 17..32
+  // outputs and of 256 for 65..128 are faster than the shortest (the latter
+  // 13.5 against 14.5 us at 2^22).
   if (pattern == OMR_NTT_PATTERN_STRIDED && count < n && !(count > 65536 && n / count <= 8))
     return run_fold<F>(d, -1, count, in, out, stream);
   if ((pattern == OMR_NTT_PATTERN_PREFIX || pattern == OMR_NTT_PATTERN_INDICES) && count <= 4096 &&
-      count < n && n / count >= 2 && d->log_n > 20)
-    return launch_prefix<F>(d, (uint32_t)count, 0, in, out, stream,
+      count < n && n / count >= 2 && (d->log_n > 20 || (count <= 256 && d->log_n >= 16))) {
+    const int logt = count > 16 && count <= 32 ? 6 : (count > 64 && count <= 128 ? 8 : 0);
+    return launch_prefix<F>(d, (uint32_t)count, logt, in, out, stream,
                             pattern == OMR_NTT_PATTERN_INDICES ? indices : nullptr);
+  }
   return run_gather<F>(d, -1, pattern, count, indices, in, out, stream);
 }
 

@@ -240,48 +240,40 @@ static bool db_lookup(int field, uint32_t log_n, uint64_t batch, int pattern, ui
   return true;
 }
 
-// Built-in heuristic (from the exhaustive tuner's timings on GB300): two
-// passes of short lines at 2^10..2^12, the wide pass where a transform splits
-// into 256-point passes only (2^24 = 256^3, and batches of 2^16 = 256^2; one
-// 2^16 transform is latency bound and takes the cluster plan), the one-launch
-// cluster plan for small or batched 2^13..2^16 transforms, else the slab pass
-// with one more pass than the fewest (Goldilocks) or the TMA two-CTA pass on
-// the balanced split (32-bit fields), else plan 0.
+// Built-in heuristic, as a full class (from timings of every plan on GB300):
+// below 2^10 one launch; up to 2^15 the one-launch cluster plan (BabyBear 2^12
+// 3.2 us back to back, two passes 5.9); 2^16 and 2^17 two TMA passes
+// (Goldilocks: three slab-plan passes), batches of 2^16 the wide pass; above,
+// the slab-plan or wide passes of the split that was the fastest.
+static int heuristic_class(int field, uint32_t log_n, uint64_t batch) {
+  constexpr int kCluster = 3, kTma = 8, kSlab = 12, kSlabMore = 14, kSlabLarge = 15, kWide = 16, kWideMore = 18;
+  const bool gl = field == GOLDILOCKS;
+  const uint64_t words = batch << log_n;
+  switch (log_n) {
+    case 10: case 11: case 12: case 13: case 14: case 15: return kCluster;
+    case 16: return batch >= 8 ? kWide : (gl ? kSlabMore : kTma);
+    case 17: return gl ? kSlabMore : kTma;
+    case 18: return gl || batch < 10 ? kTma : kSlab;
+    case 19: return gl || words < (1ull << 21) ? kTma : kSlab;
+    case 20: return gl && words >= (1ull << 22) ? kSlabMore : kSlab;
+    case 21: return gl ? kSlabMore : kSlabLarge;
+    case 22: return gl ? kSlabMore : (words >= (1ull << 24) ? kWideMore : kSlab);
+    case 23: case 24: return kWideMore;
+    default: return log_n < 10 ? 0 : (gl ? kSlabMore : kTma);
+  }
+}
+
 static int heuristic_full_plan(int field, uint32_t log_n, uint64_t batch) {
   const auto& plans = plan_table(log_n);
   if (plans.size() <= 1) return 0;
-  // 2^10..2^12: two passes of short lines on the two-CTA variant (class 10)
-  // beat the one-CTA single pass by 20-90% on GB300 (one CTA per transform
-  // leaves the GPU idle); below 2^10 the single launch stays
-  if (log_n >= 10 && log_n <= 12) {
-    const int p = full_class_plan(log_n, 4 * 2 + 2);
-    if (p >= 0) return p;
-  }
-  if (plans[0].split.size() < 2) return 0;
-  if (log_n == 24 || (log_n == 16 && batch >= 8))
-    for (int i = 0; i < (int)plans.size(); i++)
-      if (plans[i].variant == kWideVariant &&
-          std::all_of(plans[i].split.begin(), plans[i].split.end(), [](int t) { return t == 8; }))
-        return i;
-  // the one-launch cluster plan wins where latency dominates: up to 2^14, or
-  // batches of 8 and more (one cluster per transform)
-  if (log_n <= 14 || batch >= 8)
-    for (int i = 0; i < (int)plans.size(); i++)
-      if (plans[i].variant == kClusterVariant) return i;
-  // Goldilocks 2^15..2^23: the slab pass on the balanced split with one more
-  // pass (class 14)
-  if (field == GOLDILOCKS) {
-    const int p = full_class_plan(log_n, 4 * 3 + 2);
-    if (p >= 0) return p;
-  }
+  const int p = full_class_plan(log_n, heuristic_class(field, log_n, batch));
+  if (p >= 0) return p;
+  // above 2^24, where the class has no plan: the first (balanced) split,
+  // double-buffered TMA passes
   size_t nsplit = 0;
-  for (auto& p : plans)
-    if (p.variant == 0) nsplit++;
-  // 32-bit fields: variant 2 (two CTAs per SM at <= 64 registers);
-  // Goldilocks: variant 1 (double-buffered)
-  const bool narrow = field != GOLDILOCKS;
-  const int cand = (int)nsplit * (narrow ? 2 : 1);  // first (balanced) split
-  return cand < (int)plans.size() ? cand : 0;
+  for (auto& q : plans)
+    if (q.variant == 0) nsplit++;
+  return nsplit < plans.size() ? (int)nsplit : 0;
 }
 
 int planned_full_plan(int field, uint32_t log_n, uint64_t batch, bool use_learned) {

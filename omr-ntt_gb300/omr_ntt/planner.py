@@ -204,27 +204,36 @@ GATHER_CLASS = FOLD_CLASS + FULL_CLASSES
 
 def heuristic_class(p) -> int:
     """The class the planner picks without database or network (its built-in
-    rule, tuner.cu heuristic_full_plan and partial.cu partial_dispatch): two
-    passes of short lines at 2^10..2^12, the wide pass where the transform
-    splits into 256-point passes only (2^24; batches of 2^16), the cluster
-    plan for small or batched 2^13..2^16, else the TMA two-CTA pass on the
-    balanced split (32-bit fields) or the slab pass with one more pass
-    (Goldilocks); the decomposition for prefixes and index sets of <= 4096
-    outputs above 2^20, the fold for strided sets (but for more than 2^16
-    outputs of at most 8 cosets), else the full transform and a gather."""
+    rule, tuner.cu heuristic_class and partial.cu partial_dispatch): one launch
+    below 2^10, the cluster plan up to 2^15, then by size, field and batch the
+    TMA, slab-plan or wide passes of the fastest split; the decomposition for
+    prefixes and index sets of <= 256 outputs from 2^16 and of <= 4096 above
+    2^20, the fold for strided sets (but for more than 2^16 outputs of at most 8 cosets), else the full
+    transform and a gather."""
+    cluster, tma, slab, slab_more, slab_large, wide, wide_more = 3, 8, 12, 14, 15, 16, 18
+
     def full_class(log_n, batch):
-        if 10 <= log_n <= 12:
-            return 4 * 2 + 2  # two passes of short lines, TMA two-CTA variant
+        gl = p["field"] == 1
+        words = batch << log_n
         if log_n < 10:
-            return 0  # one launch
-        if log_n == 24:
-            return 4 * 4 + 2  # wide pass, 256 x 256 x 256 (one pass more than the fewest)
-        if log_n == 16 and batch >= 8:
-            return 4 * 4 + 0  # wide pass, 256 x 256
-        if 13 <= log_n <= 16 and (log_n <= 14 or batch >= 8):
-            return 3  # the one-launch cluster plan
-        # BabyBear: TMA two CTAs per SM, balanced; Goldilocks: slab, one more pass
-        return 4 * 3 + 2 if p["field"] == 1 else 4 * 2 + 0
+            return 0
+        if log_n <= 15:
+            return cluster
+        if log_n == 16:
+            return wide if batch >= 8 else (slab_more if gl else tma)
+        if log_n == 17:
+            return slab_more if gl else tma
+        if log_n == 18:
+            return tma if gl or batch < 10 else slab
+        if log_n == 19:
+            return tma if gl or words < 1 << 21 else slab
+        if log_n == 20:
+            return slab_more if gl and words >= 1 << 22 else slab
+        if log_n == 21:
+            return slab_more if gl else slab_large
+        if log_n == 22:
+            return slab_more if gl else (wide_more if words >= 1 << 24 else slab)
+        return wide_more
 
     full_cls = full_class(p["log_n"], p["batch"])
     n, s = 1 << p["log_n"], point_count(p)
@@ -232,8 +241,9 @@ def heuristic_class(p) -> int:
         return full_cls
     if p["pattern"] == "strided" and not (p["log_s"] > 16 and p["log_n"] - p["log_s"] <= 3):
         return FOLD_CLASS + full_class(p["log_s"], 1)
-    if p["pattern"] in ("contiguous", "random") and s <= 4096 and n // s >= 2 and p["log_n"] > 20:
-        return DECOMP_CLASS
+    if (p["pattern"] in ("contiguous", "random") and s <= 4096 and n // s >= 2
+            and (p["log_n"] > 20 or (s <= 256 and p["log_n"] >= 16))):
+        return DECOMP_CLASS + (1 if 16 < s <= 32 or 64 < s <= 128 else 0)
     return GATHER_CLASS + full_class(p["log_n"], 1)  # the gather runs one transform at a time
 
 

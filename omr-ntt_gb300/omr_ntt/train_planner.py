@@ -26,7 +26,7 @@ def main(argv=None):
     ap.add_argument("--train", type=int, default=1500)
     ap.add_argument("--seed", type=int, default=2025)
     ap.add_argument("--reps", type=int, default=3)
-    ap.add_argument("--epochs", type=int, default=600)
+    ap.add_argument("--epochs", type=int, default=3000)
     ap.add_argument("--lr", type=float, default=3e-3)
     ap.add_argument("--out", default=os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "data"))
     ap.add_argument("--dataset", default=None, help="reuse a collected dataset")
