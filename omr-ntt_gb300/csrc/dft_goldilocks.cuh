@@ -1,9 +1,10 @@
 // dft_goldilocks.cuh -- in-register R-point DFTs (R = 2, 4, 8, 16) over
 // Goldilocks on three-limb values.
 //
-// The Goldilocks passes are bound by the integer ALU pipe, where a canonical
-// 64-bit modular add costs seven instructions and a subtract five: the borrow
-// or carry of every butterfly is folded back at once.  Here a value of the DFT
+// On canonical words the Goldilocks passes are bound by the integer ALU pipe,
+// where a 64-bit modular add costs seven instructions and a subtract five: the
+// borrow or carry of every butterfly is folded back at once.  With this DFT the
+// ALU and the multiply pipe are equally busy.  A value of the DFT
 // is x0 + x1 2^32 + x2 2^64 with a small signed x2, so an add or subtract is
 // three instructions (one carry chain, no fold), and the fold 2^64 = 2^32 - 1
 // happens once per output.  The roots are powers of two (omega_16 = -2^60),

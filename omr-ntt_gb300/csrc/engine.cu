@@ -179,7 +179,7 @@ std::vector<PlanShape> enumerate_plans(uint32_t log_n) {
       if (v > 0 && s.size() == 1) continue;  // single-pass plans have one kernel
       out.push_back(PlanShape{s, v});
     }
-  // 2^13..2^16: the balanced two-pass plan as one launch on an 8-CTA cluster
+  // 2^13..2^16: the balanced two-pass plan as one cluster launch
   // (appended, so the other plans keep their ids)
   if (log_n >= 13 && log_n <= 16) out.push_back(PlanShape{splits[0], kClusterVariant});
   // the slab pass on every multi-pass split, and the wide pass on those with

@@ -297,9 +297,8 @@ template <class F, int MODE, int LOGT>
 constexpr bool has_wide_pass() {
   return LOGT == 8 || F::WORD == 4 || MODE == MODE_COL;
 }
-template <class F, int LOGT>
-constexpr uint64_t wide_min_tiles() {
-  return LOGT == 8 ? 1 : (F::WORD == 8 ? 2048 : (LOGT == 7 ? 256 : 512));
+constexpr uint64_t wide_min_tiles(int word, int logT) {
+  return logT == 8 ? 1 : (word == 8 ? 2048 : (logT == 7 ? 256 : 512));
 }
 
 // The wide pass (ntt_pass_wide.cuh) at 64-, 128- and 256-point lines on
@@ -313,7 +312,7 @@ int launch_wide_t(const PassArgs<F>& a, int* err, cudaStream_t stream) {
   if (a.L_lo % C || !tma_geometry_ok<F>(a, LOGT, MODE) || (a.tw_lo != nullptr) != TW) return 1;
   const uint64_t ntiles = a.L_b * (uint64_t)a.L_m * (a.L_lo / C);
   if (ntiles == 0) return OMR_NTT_OK;
-  if (ntiles < wide_min_tiles<F, LOGT>()) return 1;
+  if (ntiles < wide_min_tiles(F::WORD, LOGT)) return 1;
   int dev = 0;
   cudaGetDevice(&dev);
   CUtensorMap in_map, out_map;
@@ -653,9 +652,12 @@ int launch_pass(const omr_ntt_domain_s* d, const PassDesc& p, bool inverse, cons
   // as one table (shorter lines only where it is small against the data:
   // Goldilocks 2^22 takes 89.4 us without tables, 86.5 with this rule's and
   // 86.4 with four times larger ones)
-  const bool wide = variant == kWideVariant || (variant == kSlabVariant && p.logT < 8);
+  const uint64_t wide_tiles = p.L_b * (uint64_t)p.L_m * (p.L_lo / (uint32_t)((p.logT == 8 ? 128 : 256) / F::WORD));
+  const bool wide = p.logT == 8 ? variant == kWideVariant
+                                : (variant == kWideVariant || variant == kSlabVariant) && p.logT < 8 &&
+                                      wide_tiles >= wide_min_tiles(F::WORD, p.logT);
   const uint64_t entries = (uint64_t)p.L_lo << p.logT;
-  if (p.twiddle && p.mode == MODE_COL && wide && p.logT <= 8 && (p.L_m == 1 || p.tw_line_mul_m == 0) &&
+  if (p.twiddle && p.mode == MODE_COL && wide && (p.L_m == 1 || p.tw_line_mul_m == 0) &&
       entries <= kLineTwMaxEntries && (p.logT == 8 || entries * 4 <= d->n * p.L_b)) {
     rc = line_twiddles<F>(const_cast<omr_ntt_domain_s*>(d), inverse, p.logT, p.tw_scale, p.L_lo, may_alloc, &a.tw_tab);
     if (rc) return rc;
