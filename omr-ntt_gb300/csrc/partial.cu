@@ -93,20 +93,18 @@ __global__ void __launch_bounds__(256) fold_flat_kernel(const typename F::E* __r
 // words per load, eight loads in flight.  The grid stride is a multiple of
 // count (count a power of two <= 4096; gridDim a multiple of 4 and of
 // count / CH), so each of a thread's VW lanes stays in one column.  The CTA
-// then sums the CH = 256 VW positions of its chunk down to columns in shared
+// then sums the CH = NT VW positions of its chunk down to columns in shared
 // memory:
 //   count <= CH: one row of count column sums per CTA;
 //   count >  CH: the CTA's chunk is CH consecutive columns of one row
 //               (row = blockIdx / (count / CH)).
-constexpr int kFoldThreads = 256;
-template <class F>
-__global__ void __launch_bounds__(kFoldThreads) fold_vec_kernel(const typename F::E* __restrict__ x,
-                                                                uint64_t n, uint32_t count,
-                                                                typename F::E* __restrict__ partial) {
+template <class F, int NT>
+__global__ void __launch_bounds__(NT) fold_vec_kernel(const typename F::E* __restrict__ x, uint64_t n,
+                                                      uint32_t count, typename F::E* __restrict__ partial) {
   pdl_entry();
   using E = typename F::E;
   constexpr int VW = 16 / F::WORD;
-  constexpr int CH = kFoldThreads * VW;  // words per CTA per sweep step
+  constexpr int CH = NT * VW;  // words per CTA per sweep step
   __shared__ E red[CH];
   const uint64_t stride = (uint64_t)gridDim.x * CH;
   E acc[VW];
@@ -135,17 +133,36 @@ __global__ void __launch_bounds__(kFoldThreads) fold_vec_kernel(const typename F
   __syncthreads();
   // position p of the chunk holds column (blockIdx * CH + p) mod count
   for (uint32_t h = CH / 2; h >= count && h >= 1; h >>= 1) {
-    for (uint32_t p = threadIdx.x; p < h; p += kFoldThreads) red[p] = F::add(red[p], red[p + h]);
+    for (uint32_t p = threadIdx.x; p < h; p += NT) red[p] = F::add(red[p], red[p + h]);
     __syncthreads();
   }
   if (count <= (uint32_t)CH) {
-    for (uint32_t c = threadIdx.x; c < count; c += kFoldThreads)
+    for (uint32_t c = threadIdx.x; c < count; c += NT)
       partial[(uint64_t)blockIdx.x * count + c] = red[c];
   } else {
     const uint32_t per = count / CH;
     E* row = partial + (uint64_t)(blockIdx.x / per) * count + (uint64_t)(blockIdx.x % per) * CH;
-    for (uint32_t p = threadIdx.x; p < (uint32_t)CH; p += kFoldThreads) row[p] = red[p];
+    for (uint32_t p = threadIdx.x; p < (uint32_t)CH; p += NT) row[p] = red[p];
   }
+}
+
+// Launches the fold; *rows_out is the number of partial rows it leaves.
+template <class F, int NT>
+static int launch_fold_vec(const omr_ntt_domain_s* d, uint64_t count, const void* in, typename F::E* part,
+                           uint64_t* rows_out, cudaStream_t stream) {
+  constexpr uint64_t ch = (uint64_t)NT * (16 / F::WORD);
+  // 1024 threads per SM, a multiple of 4 (and of count / CH) CTAs, never more
+  // than the sweep needs
+  uint64_t g = (uint64_t)device_sm_count(d->device) * (1024 / NT);
+  const uint64_t need = d->n / ch;
+  if (g > need) g = need;
+  const uint64_t m = count / ch > 4 ? count / ch : 4;  // grid stride a multiple of count
+  g = g < m ? m : g & ~(m - 1);
+  const uint32_t grid = (uint32_t)g;
+  OMR_CUDA_TRY(launch_pdl(fold_vec_kernel<F, NT>, dim3(grid), dim3(NT), 0, stream,
+                          static_cast<const typename F::E*>(in), d->n, (uint32_t)count, part));
+  *rows_out = count > ch ? grid / (count / ch) : grid;
+  return OMR_NTT_OK;
 }
 
 template <class F>
@@ -166,20 +183,19 @@ static int run_fold(omr_ntt_domain_s* d, int sub_plan, uint64_t count, const voi
   if (rc) return rc;
   E* part = static_cast<E*>(buf);
   uint64_t nch = 0;
-  const int vw = 16 / (int)w;
-  const uint64_t ch = (uint64_t)kFoldThreads * vw;
-  if (count <= 4096 && d->n >= ch * 4 && !(reinterpret_cast<uintptr_t>(in) & 15)) {
-    // 16-byte loads: four CTAs per SM, a multiple of 4 (and of
-    // count / CH), never more than the sweep needs
-    uint64_t g = (uint64_t)device_sm_count(d->device) * 4;
-    const uint64_t need = d->n / ch;
-    if (g > need) g = need;
-    const uint64_t m = count / ch > 4 ? count / ch : 4;  // grid stride a multiple of count
-    g = g < m ? m : g & ~(m - 1);
-    const uint32_t grid = (uint32_t)g;
-    OMR_CUDA_TRY(launch_pdl(fold_vec_kernel<F>, dim3(grid), dim3(kFoldThreads), 0, stream, static_cast<const E*>(in), d->n,
-                            (uint32_t)count, part));
-    nch = count > ch ? grid / (count / ch) : grid;
+  constexpr uint64_t kWords = 16 / F::WORD;  // of one load
+  if (count <= 4096 && d->n >= 256 * kWords * 4 && !(reinterpret_cast<uintptr_t>(in) & 15)) {
+    // the same 1024 threads per SM as two CTAs of 512 leave half the rows to
+    // the reduction, as long as every SM gets one.  On GB300, whole calls with
+    // 512 / 256 threads: BabyBear 2^22, 16 outputs 7.7 / 8.4 us, 128 9.0 / 10.2,
+    // 512 10.2 / 10.9; Goldilocks 2^22, 256 outputs 13.6 / 15.5, 2^18 10.7 /
+    // 11.4; more outputs 9.9 / 8.7 (2^12, a row is split over CTAs either way)
+    // and BabyBear 2^18 (128 CTAs) 8.7 / 8.4.
+    if (count <= 512 && d->n >= 512 * kWords * 256)
+      rc = launch_fold_vec<F, 512>(d, count, in, part, &nch, stream);
+    else
+      rc = launch_fold_vec<F, 256>(d, count, in, part, &nch, stream);
+    if (rc) return rc;
   } else if (count <= 4096 && d->n >= 256ull * 1216) {
     const uint32_t grid = 1216;  // 8 CTAs per SM; a multiple of count / 256 for count <= 4096
     OMR_CUDA_TRY(launch_pdl(fold_flat_kernel<F>, dim3(grid), dim3(256), 0, stream, static_cast<const E*>(in), d->n,
