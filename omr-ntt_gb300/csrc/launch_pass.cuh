@@ -641,6 +641,17 @@ int line_twiddles(omr_ntt_domain_s* d, bool inverse, int logT, uint64_t tw_scale
   return OMR_NTT_OK;
 }
 
+// A capture takes no allocation: a pass that is captured before its table
+// exists keeps the chain (the same words).
+inline bool stream_capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
 template <class F>
 int launch_pass(const omr_ntt_domain_s* d, const PassDesc& p, bool inverse, const void* in,
                 void* out, bool last, cudaStream_t stream, bool may_alloc) {
@@ -659,7 +670,10 @@ int launch_pass(const omr_ntt_domain_s* d, const PassDesc& p, bool inverse, cons
   const uint64_t entries = (uint64_t)p.L_lo << p.logT;
   if (p.twiddle && p.mode == MODE_COL && wide && (p.L_m == 1 || p.tw_line_mul_m == 0) &&
       entries <= kLineTwMaxEntries && (p.logT == 8 || entries * 4 <= d->n * p.L_b)) {
-    rc = line_twiddles<F>(const_cast<omr_ntt_domain_s*>(d), inverse, p.logT, p.tw_scale, p.L_lo, may_alloc, &a.tw_tab);
+    auto* dom = const_cast<omr_ntt_domain_s*>(d);
+    rc = line_twiddles<F>(dom, inverse, p.logT, p.tw_scale, p.L_lo, false, &a.tw_tab);
+    if (!rc && !a.tw_tab && may_alloc && !stream_capturing(stream))
+      rc = line_twiddles<F>(dom, inverse, p.logT, p.tw_scale, p.L_lo, true, &a.tw_tab);
     if (rc) return rc;
   }
   const int C = tile_cols<F, 0>();
