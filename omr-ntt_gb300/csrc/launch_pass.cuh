@@ -337,13 +337,15 @@ int launch_wide_t(const PassArgs<F>& a, int* err, cudaStream_t stream) {
     r = encode_2d(&out_map, F::WORD, a.out, w, T * a.L_b, w, BC, T, sw);
   }
   if (r != CUDA_SUCCESS) return fail(OMR_NTT_ERR_CUDA, "cuTensorMapEncodeTiled (wide store) failed");
-  if constexpr (F::WORD == 8) {
-    // Goldilocks: the warp-specialised form (one CTA per SM, no CTA barrier)
-    // is 4-7% faster on GB300 (2^24 0.378 against 0.400 ms, 64 x 2^20 1.33
-    // against 1.41 ms); for the 32-bit fields it is 8-10% slower at 2^24
+  if constexpr (F::WORD == 8 && MODE == MODE_COL) {
+    // Goldilocks column passes: the warp-specialised form (one CTA per SM, no
+    // CTA barrier).  On GB300 against three CTAs an SM, us: whole transforms
+    // 64 x 2^18 217 / 239, 4 x 2^23 485 / 534; a pass of 2^24 100.0 / 99.1 and
+    // 88.0 / 87.8.  Row passes re-lay their lines and lose in it (2^24 80.5 /
+    // 73.0).  For the 32-bit fields it is 8-10% slower at 2^24.
     constexpr size_t smem = wide_ws_smem_bytes<F, LOGT>();
     static_assert(smem <= kMaxDynSmem, "warp-specialised wide pass does not fit in shared memory");
-    auto kern = ntt_wide_ws_pass<F, LOGT, MODE, INV, TW>;
+    auto kern = ntt_wide_ws_pass<F, LOGT, INV>;
     static std::atomic<int> ready[64];
     if (!ready[dev & 63].load()) {
       OMR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

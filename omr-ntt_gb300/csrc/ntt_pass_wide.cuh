@@ -31,8 +31,10 @@
 // in the buffer before the store) and two for row passes (the lines are
 // re-laid as rows in place).  Waits are bounded as in the other passes.
 // Thread 0 waits on the previous kernel of the stream (programmatic
-// dependent launch) before the first load.  Goldilocks runs the
-// warp-specialised form at the end of this file.
+// dependent launch) before the first load.  Goldilocks column
+// passes run the warp-specialised form at the end of this file; its row passes
+// are faster in three CTAs an SM, which hide each other's barriers (the 2^24
+// row pass 73.0 against 80.5 us).
 //
 // The line transform is the same split as the slab pass (ntt_pass_slab.cuh),
 // i.e. the reference's four-step decomposition
@@ -213,31 +215,6 @@ OMR_D void wide_issue_store(const CUtensorMap* map, const PassArgs<F>& a, uint64
                    buf + b * T * 128);
   }
   bulk_commit();
-}
-
-// wide_issue_load by a whole warp: a row pass's C <= 32 line copies go out
-// from C lanes at once (one thread issues a bulk copy in ~70 ns, so C = 32
-// copies from one thread take longer than the tile's compute).  The
-// expect-tx arrive (lane 0) comes first; column passes are one or two TMA
-// loads.
-template <class F, int LOGT, int MODE>
-OMR_D void wide_issue_load_warp(const CUtensorMap* map, const PassArgs<F>& a, uint64_t tile,
-                                unsigned char* buf, uint64_t* bar, int lane) {
-  using E = typename F::E;
-  constexpr int T = 1 << LOGT, C = wide_cols<F, LOGT>();
-  if constexpr (MODE == MODE_COL || wide_line_boxes<F, LOGT>()) {
-    if (lane == 0) wide_issue_load<F, LOGT, MODE>(map, a, tile, buf, bar);
-  } else {
-    static_assert(C <= 32, "one line copy a lane");
-    uint32_t g, lm;
-    uint64_t lb;
-    tile_coords<F, C>(a, tile, g, lm, lb);
-    if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)(T * C * F::WORD));
-    __syncwarp();
-    const E* src = a.in + (lb * a.is_b + lm * a.is_m + (uint64_t)(g * C) * a.is_lo);
-    if (lane < C)
-      bulk_load(buf + lane * wide_line_bytes<F, LOGT>(), src + (uint64_t)lane * a.is_lo, T * F::WORD, bar);
-  }
 }
 
 // Unit w's results (wide_lines) to the swizzled rows.
@@ -441,16 +418,14 @@ __global__ void __launch_bounds__(kWideThreads, 3)  // shared memory holds three
 }
 
 // ---------------------------------------------------------------------------
-// The same pass as one warp-specialised CTA per SM.  kWideSlots tile buffers
+// The column pass as one warp-specialised CTA per SM.  kWideSlots tile buffers
 // cycle through load -> compute -> store: a loader warp issues the TMA loads,
 // 24 consumer warps claim units (tile j, column group w) in order from a
 // shared counter, so the eight column groups of a tile run on eight warps at
 // once and every warp stays busy until the CTA's last unit, and a storer warp
 // issues each tile's TMA store and hands the buffer back.  No CTA barrier:
 // per buffer slot, `full` completes when the tile has landed, `done` when its
-// eight units are written back, `empty` when its store has read it, and for
-// row passes `rd` when its eight units have read their lines (the lines are
-// re-laid as rows in place).
+// eight units are written back, `empty` when its store has read it.
 //
 // Units are claimed in order but finish in any order, so a consumer can be
 // more than one use of its slot ahead of the loads (a slow warp holding a
@@ -458,9 +433,9 @@ __global__ void __launch_bounds__(kWideThreads, 3)  // shared memory holds three
 // others run on).  A parity wait alone would then see an old phase as done:
 // the producer publishes which tile each slot holds (`slot_tile`) before it
 // issues the load, and a consumer waits for its tile to be the slot's before
-// it waits on `full`.  `rd` and `done` are safe without that check, because
-// a unit reaches them only after its tile's load, i.e. after every unit of
-// the slot's previous tile has passed both.
+// it waits on `full`.  `done` is safe without that check, because a unit
+// reaches it only after its tile's load, i.e. after every unit of the slot's
+// previous tile has passed it.
 // 24 consumer warps (72 registers at 832 threads).  For the 32-bit fields
 // the form measured slower than the three-CTA pass with 24 consumers at 72
 // registers and with 22 at 80, so only Goldilocks launches it.
@@ -479,7 +454,7 @@ constexpr size_t wide_ws_smem_bytes() {
   return kWideSlots * (size_t)wide_buf_bytes<F, LOGT>() + wide_tab_entries<F, LOGT>() * sizeof(typename F::Tw) + 1024;
 }
 
-template <class F, int LOGT, int MODE, bool INV, bool TW>
+template <class F, int LOGT, bool INV>  // column passes
 __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
     ntt_wide_ws_pass(const __grid_constant__ CUtensorMap in_map,
                      const __grid_constant__ CUtensorMap out_map, const PassArgs<F> a, int* err) {
@@ -488,7 +463,7 @@ __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
   constexpr int C = wide_cols<F, LOGT>(), VPU = slab_vpu<F>(), S = kWideSlots;
   constexpr int BB = wide_buf_bytes<F, LOGT>();
   extern __shared__ __align__(1024) unsigned char wide_ws_smem_raw[];
-  __shared__ __align__(8) uint64_t full[S], done[S], rd[S], empty[S];
+  __shared__ __align__(8) uint64_t full[S], done[S], empty[S];
   __shared__ uint32_t unit_next;
   __shared__ volatile uint32_t slot_tile[S];  // j of the load last issued into each slot
   __shared__ volatile int abort_flag;
@@ -516,11 +491,13 @@ __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
         abort_flag = 1;
       }
       go = !abort_flag;
-      if (go) slot_tile[s] = j_load;
+      if (go) {
+        slot_tile[s] = j_load;
+        wide_issue_load<F, LOGT, MODE_COL>(&in_map, a, tile_of(j_load), base + s * BB, &full[s]);
+      }
     }
     go = __shfl_sync(0xffffffffu, go, 0);
     if (!go) return false;
-    wide_issue_load_warp<F, LOGT, MODE>(&in_map, a, tile_of(j_load), base + s * BB, &full[s], lane);
     j_load++;
     return true;
   };
@@ -529,7 +506,6 @@ __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
       for (int s = 0; s < S; s++) {
         mbar_init(&full[s], 1);
         mbar_init(&done[s], 8);
-        mbar_init(&rd[s], 8);
         mbar_init(&empty[s], 1);
         slot_tile[s] = 0xffffffffu;
       }
@@ -574,7 +550,7 @@ __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
         abort_flag = 1;
       }
       if (abort_flag) break;
-      wide_issue_store<F, LOGT, MODE>(&out_map, a, tile_of(j), base + s * BB);
+      wide_issue_store<F, LOGT, MODE_COL>(&out_map, a, tile_of(j), base + s * BB);
       if (j + S < njobs) {
         bulk_wait_read_all();
         mbar_arrive(&empty[s]);
@@ -608,21 +584,7 @@ __global__ void __launch_bounds__(wide_ws_threads<F>(), 1)
     uint64_t lb;
     tile_coords<F, C>(a, tile_of(j), g, lm, lb);
     E v[VPU][1 << wide_r1_log<LOGT>()];
-    wide_lines<F, LOGT, MODE, INV, TW>(a, buf, tab1, w, g * C, lm, v);
-    if constexpr (MODE != MODE_COL) {
-      // the rows of the output span every column group's lines: re-lay after
-      // all eight units have read theirs
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&rd[s]);
-      if (!mbar_wait_bounded(&rd[s], par)) {
-        if (lane == 0) {
-          atomicExch(err, OMR_NTT_ERR_TIMEOUT);
-          abort_flag = 1;
-        }
-        break;
-      }
-      wide_store_rows<F, LOGT>(buf, w, v);
-    }
+    wide_lines<F, LOGT, MODE_COL, INV, true>(a, buf, tab1, w, g * C, lm, v);
     fence_proxy_async();  // this thread's writes become visible to the TMA store
     __syncwarp();
     if (lane == 0) mbar_arrive(&done[s]);
