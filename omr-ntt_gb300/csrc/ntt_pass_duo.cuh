@@ -34,6 +34,7 @@
 #include <cuda.h>
 
 #include "ntt_pass_wide.cuh"
+#include "team_ring.cuh"
 
 namespace omr {
 
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(duo_teams<LOGT>() * duo_team_threads<LOGT>(),
   constexpr int C = kDuoCols, NT = duo_team_threads<LOGT>(), TEAMS = duo_teams<LOGT>(), L = (1 << LOGT) / 32;
   constexpr int NB = duo_bufs<LOGT>(), BB = duo_buf_bytes<LOGT>();
   extern __shared__ __align__(1024) unsigned char duo_smem_raw[];
-  __shared__ __align__(8) uint64_t full[NB];
+  __shared__ __align__(8) uint64_t sent[NB], full[NB];  // the buffer's load issued, landed
   __shared__ uint32_t issued[NB], landed[NB];  // loads of each buffer
   __shared__ volatile int abort_flag;
   unsigned char* base = duo_smem_raw + ((1024u - (smem_u32(duo_smem_raw) & 1023u)) & 1023u);
@@ -223,12 +224,14 @@ __global__ void __launch_bounds__(duo_teams<LOGT>() * duo_team_threads<LOGT>(),
   const auto issue = [&](uint32_t j) {
     const uint32_t b = j % NB;
     issued[b]++;
+    if (TEAMS > 1) mbar_arrive(&sent[b]);
     duo_issue_load<F, LOGT, MODE>(&in_map, a, blockIdx.x + (uint64_t)j * gridDim.x, base + b * BB, &full[b]);
   };
   if (threadIdx.x == 0) {
     prefetch_tmap(&in_map);
     prefetch_tmap(&out_map);
     for (int b = 0; b < NB; b++) {
+      mbar_init(&sent[b], 1);
       mbar_init(&full[b], 1);
       issued[b] = landed[b] = 0;
     }
@@ -246,42 +249,44 @@ __global__ void __launch_bounds__(duo_teams<LOGT>() * duo_team_threads<LOGT>(),
 
   const int team = TEAMS == 1 ? 0 : (int)(threadIdx.x / NT);
   const bool leader = threadIdx.x % NT == 0;
-  uint32_t refill = 0xffffffffu;  // (leader) the load that follows the last store's read
-  for (uint32_t j = team; j < njobs; j += TEAMS) {
-    const uint32_t b = j % NB;
-    unsigned char* s = base + b * BB;
-    if (!mbar_wait_bounded(&full[b], (j / NB) & 1)) {
+  struct Ops {  // (team_ring.cuh)
+    const CUtensorMap* out_map;
+    const PassArgs<F>& a;
+    unsigned char* base;
+    const Tw* tab;
+    uint64_t *sent, *full;
+    uint32_t* landed_;
+    volatile int* abort_flag;
+    int* err;
+    int team;
+    const decltype(issue)& issue_;
+    OMR_D uint64_t tile(uint32_t j) const { return blockIdx.x + (uint64_t)j * gridDim.x; }
+    OMR_D bool wait_issued(uint32_t b, uint32_t parity) { return mbar_wait_bounded(&sent[b], parity); }
+    OMR_D bool wait_landed(uint32_t b, uint32_t parity) { return mbar_wait_bounded(&full[b], parity); }
+    OMR_D void gave_up() {
       atomicExch(err, OMR_NTT_ERR_TIMEOUT);
-      abort_flag = 1;
-    } else if (leader) {
-      landed[b]++;
+      *abort_flag = 1;
     }
-    if (leader && refill != 0xffffffffu) {
-      bulk_wait_read_all();  // (long done: it had the wait above)
+    OMR_D void landed(uint32_t b) { landed_[b]++; }
+    OMR_D void issue(uint32_t j) {
       fence_proxy_async();
-      issue(refill);
-      refill = 0xffffffffu;
+      issue_(j);
     }
-    uint32_t g, lm;
-    uint64_t lb;
-    tile_coords<F, C>(a, blockIdx.x + (uint64_t)j * gridDim.x, g, lm, lb);
-    duo_lines<F, LOGT, MODE, INV, TW>(a, s, tab, g * C, lm, team);
-    fence_proxy_async();  // this thread's writes become visible to the TMA store
-    named_barrier(duo_team_barrier(team), NT);
-    if (abort_flag) break;
-    if (leader) {
-      duo_issue_store<F, LOGT, MODE>(&out_map, a, blockIdx.x + (uint64_t)j * gridDim.x, s);
-      if (j + NB < njobs) {
-        refill = j + NB;
-        if (NB == 1) {  // the next tile needs this buffer
-          bulk_wait_read_all();
-          fence_proxy_async();
-          issue(refill);
-          refill = 0xffffffffu;
-        }
-      }
+    OMR_D void transform(uint32_t j, uint32_t b) {
+      uint32_t g, lm;
+      uint64_t lb;
+      tile_coords<F, C>(a, tile(j), g, lm, lb);
+      duo_lines<F, LOGT, MODE, INV, TW>(a, base + b * BB, tab, g * C, lm, team);
+      fence_proxy_async();  // this thread's writes become visible to the TMA store
     }
-  }
+    OMR_D void team_barrier() { named_barrier(duo_team_barrier(team), NT); }
+    OMR_D bool aborted() { return *abort_flag != 0; }
+    OMR_D void store(uint32_t j, uint32_t b) {
+      duo_issue_store<F, LOGT, MODE>(out_map, a, tile(j), base + b * BB);
+    }
+    OMR_D void store_read() { bulk_wait_read_all(); }
+  } ops{&out_map, a, base, tab, sent, full, landed, &abort_flag, err, team, issue};
+  team_ring_run<NB, TEAMS>(ops, (uint32_t)team, leader, njobs);
   if (leader) bulk_wait_all();
   __syncthreads();
   // after a wait that gave up, loads may still be in flight
