@@ -93,6 +93,20 @@ OMR_D uint32_t duo_at(uint32_t l, uint32_t k, uint32_t ch, uint32_t c) {
 
 OMR_D void named_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
+// ... that tells all of its threads whether any of them brought `x`
+OMR_D bool named_barrier_any(int id, int threads, bool x) {
+  uint32_t any;
+  asm volatile(
+      "{.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %3, 0;\n\t"
+      "bar.red.or.pred p, %1, %2, q;\n\t"
+      "selp.u32 %0, 1, 0, p;}"
+      : "=r"(any)
+      : "r"(id), "r"(threads), "r"((uint32_t)x)
+      : "memory");
+  return any != 0;
+}
+
 template <class F, int LOGT, int MODE>
 OMR_D void duo_issue_load(const CUtensorMap* map, const PassArgs<F>& a, uint64_t tile, unsigned char* buf,
                           uint64_t* bar) {
@@ -279,8 +293,9 @@ __global__ void __launch_bounds__(duo_teams<LOGT>() * duo_team_threads<LOGT>(),
       duo_lines<F, LOGT, MODE, INV, TW>(a, base + b * BB, tab, g * C, lm, team);
       fence_proxy_async();  // this thread's writes become visible to the TMA store
     }
-    OMR_D void team_barrier() { named_barrier(duo_team_barrier(team), NT); }
-    OMR_D bool aborted() { return *abort_flag != 0; }
+    OMR_D bool team_aborted(bool mine) {
+      return named_barrier_any(duo_team_barrier(team), NT, mine || *abort_flag != 0);
+    }
     OMR_D void store(uint32_t j, uint32_t b) {
       duo_issue_store<F, LOGT, MODE>(out_map, a, tile(j), base + b * BB);
     }

@@ -16,12 +16,15 @@
 // Ops, called by every thread of a team but for those marked (leader):
 //   bool wait_issued(b, parity), wait_landed(b, parity)
 //                             bounded waits on buffer b's barriers; false: gave up
-//   void gave_up()            raise the error and the CTA's abort flag
+//   void gave_up()            raise the error and the abort flag of all teams
 //   void landed(b)            (leader) count a load of buffer b that has landed
 //   void issue(j)             (leader) start the load of tile j
 //   void transform(j, b)      transform tile j in its buffer
-//   void team_barrier()       barrier of the team
-//   bool aborted()            the abort flag
+//   bool team_aborted(mine)   barrier of the team; true for all of its threads
+//                             if any of them brought `mine` or saw the flag.
+//                             (A flag that each thread reads for itself can
+//                             differ between them, as other teams set it at any
+//                             time: some would leave and the rest wait for them.)
 //   void store(j, b)          (leader) start the store of tile j
 //   void store_read()         (leader) wait until the stores have read their buffers
 #pragma once
@@ -48,8 +51,7 @@ OMR_D void team_ring_run(Ops& op, uint32_t team, bool leader, uint32_t njobs) {
       refill = 0xffffffffu;
     }
     op.transform(j, b);
-    op.team_barrier();
-    if (op.aborted()) break;
+    if (op.team_aborted(!ok)) break;
     if (leader) {
       op.store(j, b);
       if (j + NB < njobs) {

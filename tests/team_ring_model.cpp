@@ -1,7 +1,10 @@
 // CPU threads on team_ring_run (csrc/team_ring.cuh): the warps of the teams,
 // buffers with parity barriers and a copy engine whose loads land after given
 // delays.  Prints one line for what went wrong; exit status 0 if nothing did.
-//   model NB TEAMS TILES LIMIT_MS DELAY_MS...   delay of load j; later loads 0
+//   model NB TEAMS TILES LIMIT_MS FLAG_MS DELAY_MS...
+// LIMIT_MS bounds a wait for a load; a load of a negative delay never lands (all
+// warps then have to end, with the error raised).  FLAG_MS is how much later
+// warp 1 of a team reads the abort flag than warp 0 does.
 #include <unistd.h>
 
 #include <atomic>
@@ -35,10 +38,11 @@ struct Buffer {
 };
 struct Barrier {
   int arrived = 0;
+  bool any = false, result = false;
   uint32_t round = 0;
 };
 struct Cta {
-  int nb, teams, tiles, limit_ms;
+  int nb, teams, tiles, limit_ms, flag_ms;
   std::vector<int> delay_ms;
   std::vector<Buffer> buf;
   std::vector<Barrier> team;
@@ -58,7 +62,7 @@ struct Cta {
     };
     if (d == 0)
       land();
-    else
+    else if (d > 0)
       copies.emplace_back([=, this] {
         std::this_thread::sleep_for(ms(d));
         std::lock_guard<std::mutex> lk(mu);
@@ -93,22 +97,28 @@ struct Ops {
       std::this_thread::sleep_for(std::chrono::microseconds(200));
     }
   }
-  void team_barrier() {
+  bool aborted() {
+    if (warp == 1) std::this_thread::sleep_for(ms(c.flag_ms));
+    std::lock_guard<std::mutex> lk(mu);
+    return c.abort_flag;
+  }
+  bool team_barrier(bool x) {
     std::unique_lock<std::mutex> lk(mu);
     Barrier& bar = c.team[t];
     const uint32_t round = bar.round;
+    bar.any |= x;
     if (++bar.arrived == kWarps) {
       bar.arrived = 0;
+      bar.result = bar.any;
+      bar.any = false;
       bar.round++;
       cv.notify_all();
     } else if (!cv.wait_for(lk, ms(20 * c.limit_ms + 5000), [&] { return bar.round != round; })) {
       wrong("a warp waits for ever at its team's barrier", -1, t);
     }
+    return bar.result;
   }
-  bool aborted() {
-    std::lock_guard<std::mutex> lk(mu);
-    return c.abort_flag;
-  }
+  bool team_aborted(bool mine) { return team_barrier(mine || aborted()); }
   void store(uint32_t j, uint32_t b) {
     std::lock_guard<std::mutex> lk(mu);
     if (c.buf[b].tile != (int)j) wrong("stored a buffer that holds another tile", j, c.buf[b].tile);
@@ -140,7 +150,8 @@ int main(int argc, char** argv) {
   c.teams = std::atoi(argv[2]);
   c.tiles = std::atoi(argv[3]);
   c.limit_ms = std::atoi(argv[4]);
-  for (int i = 5; i < argc; i++) c.delay_ms.push_back(std::atoi(argv[i]));
+  c.flag_ms = std::atoi(argv[5]);
+  for (int i = 6; i < argc; i++) c.delay_ms.push_back(std::atoi(argv[i]));
   c.buf.resize(c.nb);
   c.team.resize(c.teams);
   c.stored.assign(c.tiles, 0);
@@ -150,8 +161,10 @@ int main(int argc, char** argv) {
     run<1, 1>(c);
   else
     wrong("no such ring", c.nb, c.teams);
-  if (c.abort_flag) wrong("gave up", -1, 0);
+  bool lost = false;
+  for (int d : c.delay_ms) lost |= d < 0;
+  if (c.abort_flag != lost) wrong("abort flag", -1, c.abort_flag);
   for (int j = 0; j < c.tiles; j++)
-    if (c.stored[j] != 1) wrong("not stored once", j, c.stored[j]);
+    if (lost ? c.stored[j] > 1 : c.stored[j] != 1) wrong("not stored once", j, c.stored[j]);
   return 0;
 }

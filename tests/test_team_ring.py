@@ -1,6 +1,6 @@
 """The ring of tile buffers of the two-round pass (csrc/team_ring.cuh), run by
 CPU threads (team_ring_model.cpp): no team touches a buffer whose load has not
-landed, in whatever order the loads land."""
+landed, in whatever order the loads land, and every warp ends when one never does."""
 import os
 import random
 import shutil
@@ -22,9 +22,9 @@ def model(tmp_path_factory):
     return exe
 
 
-def _all(model, ring, limit_ms, delays):
-    runs = [subprocess.Popen([model, *map(str, ring), str(TILES), str(limit_ms), *map(str, d)], stdout=subprocess.PIPE,
-                             text=True) for d in delays]
+def _all(model, ring, limit_ms, delays, flag_ms=0):
+    runs = [subprocess.Popen([model, *map(str, [*ring, TILES, limit_ms, flag_ms, *d])], stdout=subprocess.PIPE, text=True)
+            for d in delays]
     return [(d, r.communicate(timeout=60)[0].strip()) for d, r in zip(delays, runs)]
 
 
@@ -37,3 +37,11 @@ def test_late_loads(model, ring):
     late += [[rng.choice([0, 0, 1, 3, 9]) for _ in range(TILES)] for _ in range(40)]
     for i in range(0, len(late), 12):
         assert [x for x in _all(model, ring, 20000, late[i:i + 12]) if x[1]] == []
+
+
+@pytest.mark.parametrize("ring", [(3, 2), (1, 1)], ids=["two-teams-three-buffers", "one-team-one-buffer"])
+@pytest.mark.parametrize("flag_ms", [0, 20, 130])
+def test_load_that_never_lands(model, ring, flag_ms):
+    """The waits give up after 100 ms, and no warp is left at a barrier, at whatever time its team reads the flag."""
+    lost = [[-1 if k == j else 0 for k in range(TILES)] for j in range(8)]
+    assert [x for x in _all(model, ring, 100, lost, flag_ms) if x[1]] == []
