@@ -77,9 +77,9 @@ struct PassArgs {
   uint32_t tw_line_mul_m;
   int has_scale;
   Tw scale;  // N^-1 for inverse transforms
-  // optional: the four-step twiddles of a wide or two-round column pass as
-  // one table [line][k] (tw_line_mul_m == 0), replacing the base * step^q
-  // chain with one table operand per output
+  // optional: the four-step twiddles of a wide column pass as one table
+  // [line][k] (tw_line_mul_m == 0), replacing the base * step^q chain with one
+  // table operand per output
   const Tw* tw_tab;
 };
 
