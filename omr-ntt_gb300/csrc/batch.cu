@@ -520,14 +520,10 @@ int omr_ntt_batch_build(omr_ntt_batch_t b) {
     batch_free_device(b);
     return fail(OMR_NTT_ERR_ALLOC, std::string("batch device state: ") + cudaGetErrorString(e));
   }
-  OMR_CUDA_TRY(cudaMemcpy(b->d_reqs, b->reqs.data(), sizeof(BatchReq) * b->reqs.size(),
-                          cudaMemcpyHostToDevice));
-  OMR_CUDA_TRY(cudaMemcpy(b->d_tasks, b->tasks.data(), sizeof(BatchTask) * b->tasks.size(),
-                          cudaMemcpyHostToDevice));
-  if (!b->idx.empty())
-    OMR_CUDA_TRY(cudaMemcpy(b->d_idx, b->idx.data(), sizeof(uint32_t) * b->idx.size(),
-                            cudaMemcpyHostToDevice));
-  OMR_CUDA_TRY(cudaMemset(b->d_err, 0, sizeof(int)));
+  OMR_CUDA_TRY(cudaMemset(b->d_err, 0, sizeof(int)));  // (ended with the uploads, in the same stream)
+  OMR_CUDA_TRY(upload(b->d_reqs, b->reqs.data(), sizeof(BatchReq) * b->reqs.size()));
+  OMR_CUDA_TRY(upload(b->d_tasks, b->tasks.data(), sizeof(BatchTask) * b->tasks.size()));
+  if (!b->idx.empty()) OMR_CUDA_TRY(upload(b->d_idx, b->idx.data(), sizeof(uint32_t) * b->idx.size()));
   OMR_CUDA_TRY(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kBatchSmem));
   int occ = 0;
@@ -621,7 +617,7 @@ int omr_ntt_batch_inject_stall(omr_ntt_batch_t b, uint32_t req) {
   DeviceGuard g(b->device);
   BatchReq r = b->reqs[req];
   r.groups0 += 1;
-  OMR_CUDA_TRY(cudaMemcpy(b->d_reqs + req, &r, sizeof(BatchReq), cudaMemcpyHostToDevice));
+  OMR_CUDA_TRY(upload(b->d_reqs + req, &r, sizeof(BatchReq)));
   return OMR_NTT_OK;
 }
 

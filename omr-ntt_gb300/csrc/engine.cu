@@ -90,8 +90,8 @@ static int build_root_tables(RootTables* out) {
   const size_t bytes = sizeof(Tw) * kRoundTableWords;
   OMR_CUDA_TRY(cudaMalloc(&df, bytes));
   OMR_CUDA_TRY(cudaMalloc(&di, bytes));
-  OMR_CUDA_TRY(cudaMemcpy(df, rf.data(), bytes, cudaMemcpyHostToDevice));
-  OMR_CUDA_TRY(cudaMemcpy(di, ri.data(), bytes, cudaMemcpyHostToDevice));
+  OMR_CUDA_TRY(upload(df, rf.data(), bytes));
+  OMR_CUDA_TRY(upload(di, ri.data(), bytes));
   out->fwd = df;
   out->inv = di;
   return OMR_NTT_OK;
@@ -357,8 +357,8 @@ static int build_domain_tables(omr_ntt_domain_s* d) {
     void *dlo = nullptr, *dhi = nullptr;
     OMR_CUDA_TRY(cudaMalloc(&dlo, sizeof(E) * nlo));
     OMR_CUDA_TRY(cudaMalloc(&dhi, sizeof(Tw) * nhi));
-    OMR_CUDA_TRY(cudaMemcpy(dlo, lo.data(), sizeof(E) * nlo, cudaMemcpyHostToDevice));
-    OMR_CUDA_TRY(cudaMemcpy(dhi, hi.data(), sizeof(Tw) * nhi, cudaMemcpyHostToDevice));
+    OMR_CUDA_TRY(upload(dlo, lo.data(), sizeof(E) * nlo));
+    OMR_CUDA_TRY(upload(dhi, hi.data(), sizeof(Tw) * nhi));
     if (dir == 0) {
       d->tw_lo_f = dlo;
       d->tw_hi_f = dhi;

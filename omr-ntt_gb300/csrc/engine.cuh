@@ -29,6 +29,14 @@ int fail(int status, const std::string& msg);
                                                cudaGetErrorString(err__));       \
   } while (0)
 
+// Host to device, complete on return.  A copy from pageable memory may return
+// with its bytes only staged, and the streams that read the tables need not be
+// ordered with the copy's.
+inline cudaError_t upload(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
+}
+
 inline int word_bytes(int field) { return field == GOLDILOCKS ? 8 : 4; }
 
 // Launch with the programmatic stream-serialisation attribute: the kernel's

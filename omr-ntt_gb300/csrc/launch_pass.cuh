@@ -409,7 +409,7 @@ int tc_operand(bool inverse, const uint16_t** out) {
       }
   void* d = nullptr;
   OMR_CUDA_TRY(cudaMalloc(&d, kTcBBytes));
-  OMR_CUDA_TRY(cudaMemcpy(d, img.data(), kTcBBytes, cudaMemcpyHostToDevice));
+  OMR_CUDA_TRY(upload(d, img.data(), kTcBBytes));
   cache[key] = d;
   *out = static_cast<const uint16_t*>(d);
   return OMR_NTT_OK;
@@ -634,7 +634,7 @@ int line_twiddles(omr_ntt_domain_s* d, bool inverse, int logT, uint64_t tw_scale
   void* dev = nullptr;
   const size_t bytes = host.size() * sizeof(Tw);
   if (cudaMalloc(&dev, bytes) != cudaSuccess) return fail(OMR_NTT_ERR_ALLOC, "line twiddle table allocation failed");
-  if (cudaMemcpy(dev, host.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+  if (upload(dev, host.data(), bytes) != cudaSuccess) {
     cudaFree(dev);
     return fail(OMR_NTT_ERR_CUDA, "line twiddle table copy failed");
   }

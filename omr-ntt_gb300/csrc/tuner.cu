@@ -492,7 +492,7 @@ int omr_ntt_tune_point(int field, uint32_t log_n, uint64_t batch, int pattern, u
     uint64_t stride = (seed * 2654435761ull) | 1ull, off = seed % n;
     for (uint64_t j = 0; j < count; j++) h[j] = (uint32_t)((off + j * stride) & (n - 1));
     if (cudaMalloc(&idx, count * 4) != cudaSuccess ||
-        cudaMemcpy(idx, h.data(), count * 4, cudaMemcpyHostToDevice) != cudaSuccess)
+        upload(idx, h.data(), count * 4) != cudaSuccess)
       rc = fail(OMR_NTT_ERR_ALLOC, "tuning indices");
   }
   for (int i = 0; !rc && i < (int)cands.size(); i++) {
