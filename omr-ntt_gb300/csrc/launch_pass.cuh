@@ -6,7 +6,9 @@
 #include <atomic>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
+#include <new>
 
 #include "engine.cuh"
 #include "ntt_pass_duo.cuh"
@@ -606,6 +608,8 @@ int make_pass_args(const omr_ntt_domain_s* d, const PassDesc& p, bool inverse, c
 // (line, k) = omega^((line * tw_scale * k) mod N) as F::Tw, line < lines.
 // Built on the host once per (domain, direction, T, tw_scale, lines) and kept
 // by the domain; with may_alloc = false only an existing table is returned.
+// *out stays null where there is none, also for want of memory: the pass then
+// runs the chain (the same words).
 constexpr uint64_t kLineTwMaxEntries = 1ull << 21;  // 16 MB of 8-byte operands at most
 
 template <class F>
@@ -622,7 +626,17 @@ int line_twiddles(omr_ntt_domain_s* d, bool inverse, int logT, uint64_t tw_scale
   }
   if (!may_alloc) return OMR_NTT_OK;
   const uint64_t p = F::p64(), w = inverse ? d->omega_inv : d->omega;
-  std::vector<Tw> host((size_t)lines << logT);
+  const size_t bytes = ((size_t)lines << logT) * sizeof(Tw);
+  void* dev = nullptr;
+  if (cudaMalloc(&dev, bytes) != cudaSuccess) {
+    cudaGetLastError();  // (answered here)
+    return OMR_NTT_OK;
+  }
+  const std::unique_ptr<Tw[]> host(new (std::nothrow) Tw[(size_t)lines << logT]);
+  if (!host) {
+    cudaFree(dev);
+    return OMR_NTT_OK;
+  }
   for (uint32_t line = 0; line < lines; line++) {
     const uint64_t step = hpowmod(w, ((uint64_t)line * tw_scale) & (d->n - 1), p);
     uint64_t t = 1;
@@ -631,10 +645,7 @@ int line_twiddles(omr_ntt_domain_s* d, bool inverse, int logT, uint64_t tw_scale
       t = hmulmod(t, step, p);
     }
   }
-  void* dev = nullptr;
-  const size_t bytes = host.size() * sizeof(Tw);
-  if (cudaMalloc(&dev, bytes) != cudaSuccess) return fail(OMR_NTT_ERR_ALLOC, "line twiddle table allocation failed");
-  if (upload(dev, host.data(), bytes) != cudaSuccess) {
+  if (upload(dev, host.get(), bytes) != cudaSuccess) {
     cudaFree(dev);
     return fail(OMR_NTT_ERR_CUDA, "line twiddle table copy failed");
   }

@@ -1,5 +1,6 @@
 """The [line][k] twiddle tables a domain builds on first use, on a fake CUDA
-runtime (line_table_model.cu): no pass reads one before its copy has ended."""
+runtime (line_table_model.cu): no pass reads one before its copy has ended, and
+a pass whose table finds no memory goes on without it."""
 import os
 import subprocess
 
@@ -26,7 +27,7 @@ def model(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("limit", [1 << 30], ids=["enough-memory"])
+@pytest.mark.parametrize("limit", [1 << 30, 1 << 20, 0], ids=["enough-memory", "too-little", "none"])
 def test_table(model, limit):
     r = subprocess.run([model, str(limit)], capture_output=True, text=True, timeout=120)
     assert (r.returncode, r.stdout) == (0, "")
