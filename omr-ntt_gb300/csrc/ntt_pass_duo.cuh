@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(duo_teams<LOGT>() * duo_team_threads<LOGT>(),
       atomicExch(err, OMR_NTT_ERR_TIMEOUT);
       *abort_flag = 1;
     }
+    OMR_D bool aborted() { return *abort_flag != 0; }
     OMR_D void landed(uint32_t b) { landed_[b]++; }
     OMR_D void issue(uint32_t j) {
       fence_proxy_async();
@@ -290,9 +291,7 @@ __global__ void __launch_bounds__(duo_teams<LOGT>() * duo_team_threads<LOGT>(),
       duo_lines<F, LOGT, MODE, INV, TW>(a, base + b * BB, tab, g * C, lm, team);
       fence_proxy_async();  // this thread's writes become visible to the TMA store
     }
-    OMR_D bool team_aborted(bool mine) {
-      return named_barrier_any(duo_team_barrier(team), NT, mine || *abort_flag != 0);
-    }
+    OMR_D bool any(bool x) { return named_barrier_any(duo_team_barrier(team), NT, x); }
     OMR_D void store(uint32_t j, uint32_t b) {
       duo_issue_store<F, LOGT, MODE>(out_map, a, tile(j), base + b * BB);
     }

@@ -102,7 +102,7 @@ struct Ops {
     std::lock_guard<std::mutex> lk(mu);
     return c.abort_flag;
   }
-  bool team_barrier(bool x) {
+  bool any(bool x) {
     std::unique_lock<std::mutex> lk(mu);
     Barrier& bar = c.team[t];
     const uint32_t round = bar.round;
@@ -118,7 +118,6 @@ struct Ops {
     }
     return bar.result;
   }
-  bool team_aborted(bool mine) { return team_barrier(mine || aborted()); }
   void store(uint32_t j, uint32_t b) {
     std::lock_guard<std::mutex> lk(mu);
     if (c.buf[b].tile != (int)j) wrong("stored a buffer that holds another tile", j, c.buf[b].tile);
