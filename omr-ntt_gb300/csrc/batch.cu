@@ -76,8 +76,9 @@ struct BatchArgs {
 // Lines per tile: 8192 (BabyBear) or 4096 (Goldilocks) words a tile, so that a
 // radix-16 round has one or two butterflies for each of the 256 threads (with
 // 2048 words, half of them idled in the rounds of 256-point lines), at least
-// 32 bytes of lines, and no more lines than the smallest request of the line
-// length has (32 lines of 32 points, 64 of 64).
+// 32 bytes of lines, and at most 32 lines of 32 points (all that a 2^10 request
+// has) or 64 of 64 (all that a 2^12 request has; the 64-point columns of a 2^11
+// request are 32 and fill half of their one tile).
 template <class F>
 constexpr int batch_cols(int logt) {
   const int cap = logt == 5 ? 32 : 64;
