@@ -243,20 +243,36 @@ static bool db_lookup(int field, uint32_t log_n, uint64_t batch, int pattern, ui
 // Built-in heuristic, as a full class (from timings of every plan on GB300):
 // below 2^10 one launch; up to 2^15 the one-launch cluster plan (BabyBear 2^12
 // 3.2 us back to back, two passes 5.9); 2^16 and 2^17 two TMA passes
-// (Goldilocks: three slab-plan passes), batches of 2^16 the wide pass; above,
-// the slab-plan or wide passes of the split that was the fastest.
+// (Goldilocks: three slab-plan passes); above, the slab-plan or wide passes of
+// the split that was the fastest.  Where batches part (us, the plan taken first):
+//   2^10, 2^11  clusters of few threads fill the SMs: cluster / two passes at
+//               100 transforms BabyBear 2^11 4.9 / 5.8, at 200 8.2 / 7.6, at 400
+//               12.5 / 8.6 (2^12: 13.0 / 14.2)
+//   2^16        32-bit fields cluster / wide at 9 7.6 / 16.3, 32 13.8 / 18.0, 48
+//               20.8 / 18.2
+//   TeddyBear   two TMA passes / slab plan at 24 x 2^18 47.4 / 60.1, 4 x 2^19 20.7 /
+//               30.0, 12 x 2^19 58.7 / 65.3, 16 x 2^19 80.4 / 74.5, 3 x 2^20 33.9 /
+//               43.1, 16 x 2^20 139 / 130; 2^21 (/ 4096 x 512) 1 35.0 / 31.9, 4
+//               81.0 / 91.9, and three passes at 6 110.6 / 136.4, 16 266.6 / 313.6
 static int heuristic_class(int field, uint32_t log_n, uint64_t batch) {
   constexpr int kCluster = 3, kTma = 8, kSlab = 12, kSlabMore = 14, kSlabLarge = 15, kWide = 16, kWideMore = 18;
-  const bool gl = field == GOLDILOCKS;
+  const bool gl = field == GOLDILOCKS, tb = field == TEDDYBEAR;
   const uint64_t words = batch << log_n;
   switch (log_n) {
-    case 10: case 11: case 12: case 13: case 14: case 15: return kCluster;
-    case 16: return batch >= 8 ? kWide : (gl ? kSlabMore : kTma);
+    case 10: case 11: return batch > 128 ? kSlabMore : kCluster;
+    case 12: case 13: case 14: case 15: return kCluster;
+    case 16:
+      if (batch < 8) return gl ? kSlabMore : kTma;
+      return gl || batch > 40 ? kWide : kCluster;
     case 17: return gl ? kSlabMore : kTma;
-    case 18: return gl || batch < 10 ? kTma : kSlab;
-    case 19: return gl || words < (1ull << 21) ? kTma : kSlab;
-    case 20: return gl && words >= (1ull << 22) ? kSlabMore : kSlab;
-    case 21: return gl ? kSlabMore : kSlabLarge;
+    case 18: return gl || batch < (tb ? 40u : 10u) ? kTma : kSlab;
+    case 19: return gl || words < (1ull << (tb ? 23 : 21)) ? kTma : kSlab;
+    case 20:
+      if (tb) return words < (1ull << 24) ? kTma : kSlab;
+      return gl && words >= (1ull << 22) ? kSlabMore : kSlab;
+    case 21:
+      if (tb && batch > 1) return batch < 6 ? kTma : kSlabMore;
+      return gl ? kSlabMore : kSlabLarge;
     case 22: return gl ? kSlabMore : (words >= (1ull << 24) ? kWideMore : kSlab);
     case 23: case 24: return kWideMore;
     default: return log_n < 10 ? 0 : (gl ? kSlabMore : kTma);

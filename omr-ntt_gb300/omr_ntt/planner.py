@@ -205,31 +205,38 @@ GATHER_CLASS = FOLD_CLASS + FULL_CLASSES
 def heuristic_class(p) -> int:
     """The class the planner picks without database or network (its built-in
     rule, tuner.cu heuristic_class and partial.cu partial_dispatch): one launch
-    below 2^10, the cluster plan up to 2^15, then by size, field and batch the
-    TMA, slab-plan or wide passes of the fastest split; the decomposition for
+    below 2^10, the cluster plan up to 2^15 (but for large batches of the
+    smallest), then by size, field and batch the cluster plan or the TMA, slab-plan
+    or wide passes of the fastest split; the decomposition for
     prefixes and index sets of <= 256 outputs from 2^16 and of <= 4096 above
     2^20, the fold for strided sets (but for more than 2^16 outputs of at most 8 cosets), else the full
     transform and a gather."""
     cluster, tma, slab, slab_more, slab_large, wide, wide_more = 3, 8, 12, 14, 15, 16, 18
 
     def full_class(log_n, batch):
-        gl = p["field"] == 1
+        gl, tb = p["field"] == 1, p["field"] == 3
         words = batch << log_n
         if log_n < 10:
             return 0
         if log_n <= 15:
-            return cluster
+            return slab_more if log_n <= 11 and batch > 128 else cluster
         if log_n == 16:
-            return wide if batch >= 8 else (slab_more if gl else tma)
+            if batch < 8:
+                return slab_more if gl else tma
+            return wide if gl or batch > 40 else cluster
         if log_n == 17:
             return slab_more if gl else tma
         if log_n == 18:
-            return tma if gl or batch < 10 else slab
+            return tma if gl or batch < (40 if tb else 10) else slab
         if log_n == 19:
-            return tma if gl or words < 1 << 21 else slab
+            return tma if gl or words < 1 << (23 if tb else 21) else slab
         if log_n == 20:
+            if tb:
+                return tma if words < 1 << 24 else slab
             return slab_more if gl and words >= 1 << 22 else slab
         if log_n == 21:
+            if tb and batch > 1:
+                return tma if batch < 6 else slab_more
             return slab_more if gl else slab_large
         if log_n == 22:
             return slab_more if gl else (wide_more if words >= 1 << 24 else slab)
