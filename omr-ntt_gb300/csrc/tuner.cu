@@ -303,6 +303,18 @@ int planned_full_plan(int field, uint32_t log_n, uint64_t batch, bool use_learne
   return heuristic_full_plan(field, log_n, batch);
 }
 
+// At 2^21 the plan that is the fastest by itself in the 32-bit fields (4096 x 512)
+// is not before the gather of a prefix or a strided set: us with it / with 2048 x
+// 1024, prefix of 60000 BabyBear 29.7 / 22.7, KoalaBear 29.8 / 22.7, TeddyBear
+// 45.3 / 31.2, of 5000 BabyBear 24.0 / 21.8, 2^18 strided 30.4 / 27.6; but 60000
+// random indices 24.4 / 28.0.  At the other sizes the transform's plan is within
+// 15% of the best.
+int planned_gather_plan(int field, uint32_t log_n, int pattern) {
+  const bool other = field != GOLDILOCKS && log_n == 21 && pattern != OMR_NTT_PATTERN_INDICES;
+  const int p = other ? full_class_plan(log_n, 12) : -1;  // balanced, slab
+  return p >= 0 ? p : planned_full_plan(field, log_n, 1);
+}
+
 // Planner choice for a partial request: database, learned selector, else 0
 // (the caller's built-in heuristic).
 int planned_partial(int field, uint32_t log_n, int pattern, uint64_t count, int* strategy,

@@ -251,7 +251,9 @@ def heuristic_class(p) -> int:
     if (p["pattern"] in ("contiguous", "random") and s <= 4096 and n // s >= 2
             and (p["log_n"] > 20 or (s <= 256 and p["log_n"] >= 16))):
         return DECOMP_CLASS + (1 if 16 < s <= 32 or 64 < s <= 128 else 0)
-    return GATHER_CLASS + full_class(p["log_n"], 1)  # the gather runs one transform at a time
+    # the gather runs one transform at a time
+    other = p["field"] != 1 and p["log_n"] == 21 and p["pattern"] != "random"
+    return GATHER_CLASS + (slab if other else full_class(p["log_n"], 1))
 
 
 def regret(T, best, choice):
