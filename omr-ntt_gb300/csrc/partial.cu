@@ -190,8 +190,10 @@ static int run_fold(omr_ntt_domain_s* d, int sub_plan, uint64_t count, const voi
     // 512 / 256 threads: BabyBear 2^22, 16 outputs 7.7 / 8.4 us, 128 9.0 / 10.2,
     // 512 10.2 / 10.9; Goldilocks 2^22, 256 outputs 13.6 / 15.5, 2^18 10.7 /
     // 11.4; more outputs 9.9 / 8.7 (2^12, a row is split over CTAs either way)
-    // and BabyBear 2^18 (128 CTAs) 8.7 / 8.4.
-    if (count <= 512 && d->n >= 512 * kWords * 256)
+    // and BabyBear 2^18 (128 CTAs) 8.7 / 8.4.  Fewer than 16 outputs of the fields
+    // whose additions are the dearer: Goldilocks 2^22, 8 outputs 9.9 / 9.4, 2^24, one
+    // 28.6 / 27.9, TeddyBear 2^24, 8 17.6 / 17.1 (BabyBear 2^22, 8 outputs 0.94 : 1).
+    if (count <= 512 && (F::SMALL || count >= 16) && d->n >= 512 * kWords * 256)
       rc = launch_fold_vec<F, 512>(d, count, in, part, &nch, stream);
     else
       rc = launch_fold_vec<F, 256>(d, count, in, part, &nch, stream);
