@@ -362,6 +362,11 @@ inline int launch_reduce_rows(const typename F::E* partial, uint64_t rows, uint6
   return OMR_NTT_OK;
 }
 
+// Returns 1 ("not taken") where a few CTAs would run a second tile after all the
+// others, with many outputs' sums behind each tile, in the fields of the longer
+// arithmetic: 512 tiles on 456 slots, 200 outputs, wide / plain kernel on GB300
+// TeddyBear 2^22 23.6 / 21.9 us, Goldilocks 2^21 21.2 / 18.0 (BabyBear 2^22 15.8 /
+// 16.7; TeddyBear 2^22, 100 outputs 19.7 / 20.2, 2^23, 1024 tiles, 34.5 / 38.6).
 template <class F, int LOGT>
 inline int launch_prefix_wide(omr_ntt_domain_s* d, PassArgs<F> a, uint32_t m, const uint32_t* idx, int dev,
                               void* out, cudaStream_t stream) {
@@ -377,13 +382,14 @@ inline int launch_prefix_wide(omr_ntt_domain_s* d, PassArgs<F> a, uint32_t m, co
     occ_cache[dev & 63] = occ < 1 ? 1 : occ;
     occ = occ_cache[dev & 63];
   }
+  const uint32_t groups = a.L_lo / C;
+  uint32_t grid = (uint32_t)device_sm_count(dev) * (uint32_t)occ;
+  if (!F::SMALL && m > 128 && groups > grid && 4 * (uint64_t)groups < 5 * (uint64_t)grid) return 1;
+  if (grid > groups) grid = groups;
   CUtensorMap map;
   if (encode_2d(&map, F::WORD, a.in, a.L_lo, T, a.L_lo, C / wide_boxes<LOGT>(), T, CU_TENSOR_MAP_SWIZZLE_128B) !=
       CUDA_SUCCESS)
     return fail(OMR_NTT_ERR_CUDA, "cuTensorMapEncodeTiled (decomposition) failed");
-  const uint32_t groups = a.L_lo / C;
-  uint32_t grid = (uint32_t)device_sm_count(dev) * (uint32_t)occ;
-  if (grid > groups) grid = groups;
   void* part = nullptr;
   const int rc = domain_scratch(d, stream, (size_t)grid * m * sizeof(E), &part, 1);
   if (rc) return rc;
@@ -429,8 +435,10 @@ inline int launch_prefix_t(omr_ntt_domain_s* d, uint32_t m, const uint32_t* idx,
   a.tw_line_mul_m = 0;
   // whole tiles of columns and TMA's alignment: the wide form
   if constexpr (LOGT >= 6 && LOGT <= 8)
-    if (a.L_lo % wide_cols<F, LOGT>() == 0 && !(reinterpret_cast<uintptr_t>(in) & 15))
-      return launch_prefix_wide<F, LOGT>(d, a, m, idx, dev, out, stream);
+    if (a.L_lo % wide_cols<F, LOGT>() == 0 && !(reinterpret_cast<uintptr_t>(in) & 15)) {
+      const int rc = launch_prefix_wide<F, LOGT>(d, a, m, idx, dev, out, stream);
+      if (rc != 1) return rc;
+    }
   const uint32_t groups = (a.L_lo + C - 1) / C;
   uint32_t grid = (uint32_t)device_sm_count(dev) * (uint32_t)occ;
   if (grid > groups) grid = groups;
