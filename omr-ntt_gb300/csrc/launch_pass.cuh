@@ -609,7 +609,25 @@ int make_pass_args(const omr_ntt_domain_s* d, const PassDesc& p, bool inverse, c
 // Built on the host once per (domain, direction, T, tw_scale, lines) and kept
 // by the domain; with may_alloc = false only an existing table is returned.
 // *out stays null where there is none, also for want of memory: the pass then
-// runs the chain (the same words).
+// runs the chain (the same words).  It is built inside a transform call that
+// may otherwise do nothing but launch kernels, so a capture under way on
+// another stream must not notice: in the relaxed mode of this thread an
+// allocation is not that capture's business, and the copy has a stream of its
+// own (the legacy stream would draw in every blocking one).
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+inline cudaError_t upload_apart(void* dst, const void* src, size_t bytes) {
+  cudaStream_t s = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return e;
+  e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+  const cudaError_t ended = cudaStreamSynchronize(s);
+  cudaStreamDestroy(s);
+  return e == cudaSuccess ? ended : e;
+}
 constexpr uint64_t kLineTwMaxEntries = 1ull << 21;  // 16 MB of 8-byte operands at most
 
 template <class F>
@@ -627,6 +645,7 @@ int line_twiddles(omr_ntt_domain_s* d, bool inverse, int logT, uint64_t tw_scale
   if (!may_alloc) return OMR_NTT_OK;
   const uint64_t p = F::p64(), w = inverse ? d->omega_inv : d->omega;
   const size_t bytes = ((size_t)lines << logT) * sizeof(Tw);
+  const RelaxedCapture beside;
   void* dev = nullptr;
   if (cudaMalloc(&dev, bytes) != cudaSuccess) {
     cudaGetLastError();  // (answered here)
@@ -645,7 +664,7 @@ int line_twiddles(omr_ntt_domain_s* d, bool inverse, int logT, uint64_t tw_scale
       t = hmulmod(t, step, p);
     }
   }
-  if (upload(dev, host.get(), bytes) != cudaSuccess) {
+  if (upload_apart(dev, host.get(), bytes) != cudaSuccess) {
     cudaFree(dev);
     return fail(OMR_NTT_ERR_CUDA, "line twiddle table copy failed");
   }

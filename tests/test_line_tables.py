@@ -1,6 +1,7 @@
 """The [line][k] twiddle tables a domain builds on first use, on a fake CUDA
-runtime (line_table_model.cu): no pass reads one before its copy has ended, and
-a pass whose table finds no memory goes on without it."""
+runtime (line_table_model.cu): no pass reads one before its copy has ended, a
+pass whose table finds no memory goes on without it, and a capture under way
+on another stream is left alone."""
 import os
 import subprocess
 
