@@ -23,10 +23,10 @@
 // pattern takes 43 us with the slab pass's 16-byte rows, 27 us with 64-byte
 // rows on GB300).  A 1024-point tile takes 64 KB and 512 threads: two teams in
 // one CTA an SM share three buffers, so the tile after the two in work lands
-// meanwhile (BabyBear 64 x 2^20: 291 us; with one buffer in each of two CTAs
-// 356, with 32-byte rows 326, on the slab and TMA passes 433-450).  A
+// meanwhile (BabyBear 64 x 2^20: 287-289 us; with one buffer in each of two
+// CTAs 356, with 32-byte rows 326, on the slab and TMA passes 433-450).  A
 // 512-point tile takes 32 KB and 256 threads, four single-buffered CTAs an SM
-// (64 x 2^18: 89 us; TMA pass 104).  Waits are bounded as in the other passes.
+// (64 x 2^18: 86 us; TMA pass 104).  Waits are bounded as in the other passes.
 //
 // The line transform is the reference's four-step decomposition
 // (src/encoders/winterfell_four_step.rs:31-81) within a line.
