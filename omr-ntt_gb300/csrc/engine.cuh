@@ -102,7 +102,7 @@ int default_plan(int field, uint32_t log_n, uint64_t batch);
 // selector, whose first evaluation allocates its device buffers.
 int planned_full_plan(int field, uint32_t log_n, uint64_t batch, bool use_learned = true);
 // The full transform's plan behind a gather (tuner.cu).
-int planned_gather_plan(int field, uint32_t log_n, int pattern);
+int planned_gather_plan(int field, uint32_t log_n, int pattern, uint64_t count);
 // One-launch transform of a two-pass plan on a thread-block cluster (ntt_cluster.cu):
 // 0 launched, 1 not available for this shape (run the passes), < 0 error.
 int launch_cluster_transform(const omr_ntt_domain_s* d, const PassList& ps,

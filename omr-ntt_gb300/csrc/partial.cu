@@ -223,7 +223,7 @@ static int run_gather(omr_ntt_domain_s* d, int plan, int pattern, uint64_t count
   void* full = nullptr;
   int rc = domain_scratch(d, stream, (size_t)d->n * sizeof(E), &full, 1);
   if (rc) return rc;
-  if (plan < 0) plan = planned_gather_plan(d->field, d->log_n, pattern);
+  if (plan < 0) plan = planned_gather_plan(d->field, d->log_n, pattern, count);
   rc = run_transform(d, plan, false, in, full, 1, stream);
   if (rc) return rc;
   unsigned blocks = (unsigned)((count + 255) / 256);

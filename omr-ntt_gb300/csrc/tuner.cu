@@ -304,14 +304,19 @@ int planned_full_plan(int field, uint32_t log_n, uint64_t batch, bool use_learne
 }
 
 // At 2^21 the plan that is the fastest by itself in the 32-bit fields (4096 x 512)
-// is not before the gather of a prefix or a strided set: us with it / with 2048 x
-// 1024, prefix of 60000 BabyBear 29.7 / 22.7, KoalaBear 29.8 / 22.7, TeddyBear
-// 45.3 / 31.2, of 5000 BabyBear 24.0 / 21.8, 2^18 strided 30.4 / 27.6; but 60000
-// random indices 24.4 / 28.0.  At the other sizes the transform's plan is within
-// 15% of the best.
-int planned_gather_plan(int field, uint32_t log_n, int pattern) {
-  const bool other = field != GOLDILOCKS && log_n == 21 && pattern != OMR_NTT_PATTERN_INDICES;
-  const int p = other ? full_class_plan(log_n, 12) : -1;  // balanced, slab
+// is not before a gather: us with it / with 2048 x 1024 (slab plan), prefix of
+// 60000 BabyBear 29.7 / 22.7, KoalaBear 29.8 / 22.7, of 5000 BabyBear 24.0 / 21.8,
+// 2^18 strided 30.4 / 27.6, random indices KoalaBear 5000 24.3 / 22.2, 45000 24.4 /
+// 22.5, but 60000 24.4 / 28.0.  TeddyBear with it / on two TMA passes: prefix of
+// 20000 43.3 / 27.0, random 5000 34.5 / 27.0, 20000 34.6 / 29.9, 45000 35.1 / 33.7,
+// 65536 35.2 / 35.4 (128 x 128 x 128, the fastest by itself in the shipped
+// database, 39.8).  At the other sizes the transform's plan is within 15% of the best.
+int planned_gather_plan(int field, uint32_t log_n, int pattern, uint64_t count) {
+  int p = -1;
+  if (log_n == 21 && field == TEDDYBEAR)
+    p = full_class_plan(log_n, 8);  // balanced, TMA
+  else if (log_n == 21 && field != GOLDILOCKS && (pattern != OMR_NTT_PATTERN_INDICES || count <= 49152))
+    p = full_class_plan(log_n, 12);  // balanced, slab
   return p >= 0 ? p : planned_full_plan(field, log_n, 1);
 }
 

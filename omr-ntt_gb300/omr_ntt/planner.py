@@ -252,8 +252,11 @@ def heuristic_class(p) -> int:
             and (p["log_n"] > 20 or (s <= 256 and p["log_n"] >= 16))):
         return DECOMP_CLASS + (1 if 16 < s <= 32 or 64 < s <= 128 else 0)
     # the gather runs one transform at a time
-    other = p["field"] != 1 and p["log_n"] == 21 and p["pattern"] != "random"
-    return GATHER_CLASS + (slab if other else full_class(p["log_n"], 1))
+    if p["log_n"] == 21 and p["field"] == 3:
+        return GATHER_CLASS + tma
+    if p["log_n"] == 21 and p["field"] != 1 and (p["pattern"] != "random" or s <= 49152):
+        return GATHER_CLASS + slab
+    return GATHER_CLASS + full_class(p["log_n"], 1)
 
 
 def regret(T, best, choice):

@@ -12,9 +12,9 @@ every batch in (batch / 2, batch], so a plan is judged at both ends of that
 range, by its times over the fastest there (batch 1 alone: its time).
 `planner.install_default()` loads the file beside the learned selector: the
 database is consulted first, so plan = -1 -- and the full transform behind a
-partial output's gather (but prefixes and strided sets at 2^21 of the 32-bit
-fields, where another plan is faster) -- runs the measured-best plan for these shapes, and the network
-plans the rest (partial outputs, other batch sizes).
+partial output's gather (but at 2^21 of the 32-bit fields, where another plan
+is faster before one) -- runs the measured-best plan for these shapes, and the
+network plans the rest (partial outputs, other batch sizes).
 """
 from __future__ import annotations
 

@@ -41,11 +41,15 @@ def test_rule(field, log_n, batch, plan):
     assert passes(field, log_n, -1, batch) == passes(field, log_n, i.value, batch)
 
 
-@pytest.mark.parametrize("field,log_n,plan", [(KoalaBear, 21, "2048x1024 slab"), (TeddyBear, 21, "2048x1024 slab"),
-                                              (TeddyBear, 20, "1024x1024 tma2cta")], ids=str)
-def test_plan_behind_a_gather(field, log_n, plan):
-    p = {"field": field.id, "log_n": log_n, "log_s": 16, "pattern": "contiguous", "batch": 1}
+@pytest.mark.parametrize("field,log_n,pattern,log_s,plan",
+                         [(KoalaBear, 21, "contiguous", 16, "2048x1024 slab"), (KoalaBear, 21, "random", 15, "2048x1024 slab"),
+                          (KoalaBear, 21, "random", 16, "4096x512 slab"), (TeddyBear, 21, "contiguous", 16, "2048x1024 tma2cta"),
+                          (TeddyBear, 21, "random", 13, "2048x1024 tma2cta"), (TeddyBear, 21, "random", 16, "2048x1024 tma2cta"),
+                          (TeddyBear, 20, "contiguous", 16, "1024x1024 tma2cta")],
+                         ids=lambda v: str(getattr(v, "name", v)).replace(" ", "-"))
+def test_plan_behind_a_gather(field, log_n, pattern, log_s, plan):
+    p = {"field": field.id, "log_n": log_n, "log_s": log_s, "pattern": pattern, "batch": 1}
     s, i = ctypes.c_int(), ctypes.c_int()
-    assert L.omr_ntt_plan_class_candidate(field.id, log_n, 0, 1 << 16, P.heuristic_class(p), ctypes.byref(s),
-                                          ctypes.byref(i)) == 1
+    assert L.omr_ntt_plan_class_candidate(field.id, log_n, P.PATTERN_ID[pattern], 1 << log_s, P.heuristic_class(p),
+                                          ctypes.byref(s), ctypes.byref(i)) == 1
     assert s.value == 3 and omr_ntt.plan_describe(field, log_n, i.value) == "four-step " + plan
