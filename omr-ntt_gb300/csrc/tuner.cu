@@ -247,7 +247,10 @@ static bool db_lookup(int field, uint32_t log_n, uint64_t batch, int pattern, ui
 // the split that was the fastest.  Where batches part (us, the plan taken first):
 //   2^10, 2^11  clusters of few threads fill the SMs: cluster / two passes at
 //               100 transforms BabyBear 2^11 4.9 / 5.8, at 200 8.2 / 7.6, at 400
-//               12.5 / 8.6 (2^12: 13.0 / 14.2)
+//               12.5 / 8.6
+//   2^12        the 31-bit fields where the two passes' tiles fill whole waves: 288
+//               9.8 / 9.3, 304 11.4 / 9.6, but 305 11.4 / 13.6, 420 13.3 / 14.2;
+//               440 14.7 / 14.2, 512 16.6 / 13.9
 //   2^16        32-bit fields cluster / wide at 9 7.6 / 16.3, 32 13.8 / 18.0, 48
 //               20.8 / 18.2
 //   TeddyBear   two TMA passes / slab plan at 24 x 2^18 47.4 / 60.1, 4 x 2^19 20.7 /
@@ -260,7 +263,8 @@ static int heuristic_class(int field, uint32_t log_n, uint64_t batch) {
   const uint64_t words = batch << log_n;
   switch (log_n) {
     case 10: case 11: return batch > 128 ? kSlabMore : kCluster;
-    case 12: case 13: case 14: case 15: return kCluster;
+    case 12: return field != TEDDYBEAR && !gl && ((batch > 256 && batch <= 304) || batch > 432) ? kSlabMore : kCluster;
+    case 13: case 14: case 15: return kCluster;
     case 16:
       if (batch < 8) return gl ? kSlabMore : kTma;
       return gl || batch > 40 ? kWide : kCluster;

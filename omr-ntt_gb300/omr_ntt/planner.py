@@ -205,7 +205,7 @@ GATHER_CLASS = FOLD_CLASS + FULL_CLASSES
 def heuristic_class(p) -> int:
     """The class the planner picks without database or network (its built-in
     rule, tuner.cu heuristic_class and partial.cu partial_dispatch): one launch
-    below 2^10, the cluster plan up to 2^15 (but for large batches of the
+    below 2^10, the cluster plan up to 2^15 (but for some large batches of the
     smallest), then by size, field and batch the cluster plan or the TMA, slab-plan
     or wide passes of the fastest split; the decomposition for
     prefixes and index sets of <= 256 outputs from 2^16 and of <= 4096 above
@@ -219,7 +219,9 @@ def heuristic_class(p) -> int:
         if log_n < 10:
             return 0
         if log_n <= 15:
-            return slab_more if log_n <= 11 and batch > 128 else cluster
+            two = batch > 128 if log_n <= 11 else (
+                log_n == 12 and not gl and not tb and (256 < batch <= 304 or batch > 432))
+            return slab_more if two else cluster
         if log_n == 16:
             if batch < 8:
                 return slab_more if gl else tma

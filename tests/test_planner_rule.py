@@ -14,7 +14,9 @@ from omr_ntt.fields import KoalaBear, TeddyBear
 L = _lib.lib()
 
 POINTS = [(KoalaBear, 10, 128, "32x32 cluster"), (KoalaBear, 10, 129, "32x32 slab"), (KoalaBear, 11, 100, "64x32 cluster"),
-          (KoalaBear, 11, 400, "64x32 slab"), (TeddyBear, 11, 400, "64x32 slab"), (KoalaBear, 12, 400, "64x64 cluster"),
+          (KoalaBear, 11, 400, "64x32 slab"), (TeddyBear, 11, 400, "64x32 slab"), (KoalaBear, 12, 256, "64x64 cluster"), (KoalaBear, 12, 304, "64x64 slab"),
+          (KoalaBear, 12, 305, "64x64 cluster"), (KoalaBear, 12, 512, "64x64 slab"), (TeddyBear, 12, 304, "64x64 cluster"),
+          (KoalaBear, 12, 400, "64x64 cluster"),
           (KoalaBear, 16, 7, "256x256 tma2cta"), (KoalaBear, 16, 8, "256x256 cluster"),
           (TeddyBear, 16, 40, "256x256 cluster"), (KoalaBear, 16, 41, "256x256 wide"),
           (KoalaBear, 18, 24, "512x512 slab"), (TeddyBear, 18, 24, "512x512 tma2cta"), (TeddyBear, 18, 40, "512x512 slab"),
