@@ -269,6 +269,7 @@ def regret(T, best, choice):
 DATA_DIR = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "data")
 DEFAULT_NETWORK = os.path.join(DATA_DIR, "planner_mlp.bin")
 DEFAULT_DB = os.path.join(DATA_DIR, "planner_full.db")
+DEFAULT_PARTIAL_DB = os.path.join(DATA_DIR, "planner_partial.db")
 _default = None
 
 
@@ -276,12 +277,14 @@ def install_default(path: str = DEFAULT_NETWORK, db: str | None = DEFAULT_DB):
     """Load the network trained on GB300 and make it the planner's learned
     selector (plan = -1 and the partial entry points then use it), and load
     the database of exhaustively tuned full-transform plans (`tune_full`),
-    which the planner consults before the network."""
+    which the planner consults before the network; with the shipped database
+    also that of partial outputs (`tune_partial`)."""
     global _default
-    if db and os.path.exists(db):
-        n = lib().omr_ntt_planner_load(db.encode())
-        if n < 0:
-            check(n)
+    for path_db in (db, DEFAULT_PARTIAL_DB if db == DEFAULT_DB else None):
+        if path_db and os.path.exists(path_db):
+            n = lib().omr_ntt_planner_load(path_db.encode())
+            if n < 0:
+                check(n)
     h = ctypes.c_void_p()
     check(lib().omr_ntt_mlp_load(path.encode(), ctypes.byref(h)))
     check(lib().omr_ntt_mlp_install(h))

@@ -13,8 +13,9 @@ range, by its times over the fastest there (batch 1 alone: its time).
 `planner.install_default()` loads the file beside the learned selector: the
 database is consulted first, so plan = -1 -- and the full transform behind a
 partial output's gather (but at 2^21 of the 32-bit fields, where another plan
-is faster before one) -- runs the measured-best plan for these shapes, and the
-network plans the rest (partial outputs, other batch sizes).
+is faster before one) -- runs the measured-best plan for these shapes. Partial
+outputs have a file of their own (`tune_partial`), and the network plans the
+rest (larger counts, other batch sizes).
 """
 from __future__ import annotations
 
